@@ -226,8 +226,8 @@ def _index(case, seed):
 def _probe_weights(ix, case, h=512, beta=40.0):
     """W1, b1, W2, b2, W3, b3 of a network whose scores are beta (q.c - |c|^2 / 2), written
     with gelu(a) - gelu(-a) = a: what training on these mixtures converges to."""
-    g = _gen(case["d"] * 31 + h, 7)
-    s = 4.0 * torch.linalg.qr(torch.randn(h // 2, case["d"], generator=g, device="cuda"))[0]
+    g = torch.Generator().manual_seed(case["d"] * 31 + h)
+    s = 4.0 * torch.linalg.qr(torch.randn(h // 2, case["d"], generator=g))[0].cuda()
     proj = s @ s.T / 16.0
     w3 = beta * ix["coarse"] @ s.T / 16.0
     zero = torch.zeros(h, device="cuda")

@@ -15,9 +15,17 @@
 // correctly rounded operation on two floats, so one float subtraction gives the
 // same bits.
 //
-// One warp per point: the residual and the running vocab sit in shared memory,
-// the 32 lanes split the 256 codewords of a subspace and reduce (value, index)
-// to the smallest value with the lowest index; lane 0 runs the two offset sums.
+// Subspaces of up to 8 dimensions run in three kernels, parallel over what the float order
+// leaves free:
+//   k_encode      (point, subspace) pairs: a thread measures four points against the 256
+//                 codewords of one subspace, which sit in shared memory and are read by
+//                 broadcast; the second quantizer's residual is formed again from x, the
+//                 cell and the filter code, so nothing but codes goes through memory;
+//   k_encode_1d   a second quantizer of one-dimensional subspaces (the default): per value a
+//                 search in the sorted codewords and the exact test of the few whose
+//                 rounded distance can be the smallest, instead of all 256;
+//   k_offsets     one thread per point: the two sequential offset sums.
+// Wider subspaces: k_puck_assign, one warp per point, the 32 lanes splitting the codewords.
 #include <cuda_runtime.h>
 
 #include <cfloat>
@@ -52,6 +60,7 @@ struct AssignParams {
     int* err;                   // set to 1 for a cell id out of range
     uint64_t n;
     uint32_t d, C, F, fnsq, flsq, pnsq, plsq, stride;  // stride: shared floats per warp
+    float one;                  // 1.0f (k_encode)
 };
 
 // One quantizer's pass over the residual r (shared memory); codes to cs (shared) and out.
@@ -141,6 +150,322 @@ __global__ __launch_bounds__(kAssignWarps * 32) void k_puck_assign(AssignParams 
     }
 }
 
+// ---------------------------------------------------------------- two floats at a time
+// The packed forms round each half like the scalar instruction. A packed product feeding a
+// packed sum is contracted to one rounding by the assembler, .rn or not; where the product
+// has to be rounded by itself the sum is written as a * one + b with a `one` (1, 1) that it
+// cannot see (a kernel argument).
+__device__ __forceinline__ uint64_t f2_pack(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void f2_unpack(uint64_t v, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// Residual value of dimension t of point i in cell (c, f): x - coarse - fine, and for the
+// second quantizer less the filter codeword's value.
+template <bool SECOND>
+__device__ __forceinline__ float residual(const AssignParams& p, uint64_t i, uint32_t c, uint32_t f,
+                                          uint32_t t) {
+    float r = __fsub_rn(__fsub_rn(__ldg(p.base + i * p.d + t), __ldg(p.coarse + (uint64_t)c * p.d + t)),
+                        __ldg(p.fine + (uint64_t)f * p.d + t));
+    if (SECOND) {
+        const uint32_t fk = t / p.flsq;
+        const uint32_t code = p.f_codes[i * p.fnsq + fk];
+        r = __fsub_rn(r, __ldg(p.fcb + ((uint64_t)fk * 256 + code) * p.flsq + (t - fk * p.flsq)));
+    }
+    return r;
+}
+
+// Codes of subspace blockIdx.y. Bound by instruction issue: per (point, codeword) LSQ
+// products, LSQ - 1 sums, (|r|^2 + |w|^2) and the subtraction of 2 dot (one fused step: the
+// doubling is exact, so it rounds once like the reference's), two points per instruction,
+// and one minimum. The index is not carried along: codewords go in groups of 8, the first
+// group that lowers the minimum is kept, and its 8 values are formed once more to find the
+// first that equals it. @ENCODE@
+constexpr int kEncThreads = 256;
+constexpr int kEncPairs = 2;  // pairs of points per thread
+template <int LSQ, bool SECOND>
+__global__ __launch_bounds__(kEncThreads) void k_encode(AssignParams p) {
+    constexpr int STR = (LSQ + 2) / 2 * 2;  // 8-byte slots per codeword: values twice, norm twice
+    __shared__ __align__(16) uint64_t sw[256 * STR];
+    const uint32_t k = blockIdx.y;
+    const int tid = threadIdx.x;
+    {
+        const float* cb = (SECOND ? p.pcb : p.fcb) + ((uint64_t)k * 256 + tid) * LSQ;
+        const float wn = (SECOND ? p.pcb_norm : p.fcb_norm)[(uint64_t)k * 256 + tid];
+#pragma unroll
+        for (int t = 0; t < LSQ; ++t) {
+            const float w = __ldg(cb + t);
+            sw[tid * STR + t] = f2_pack(w, w);
+        }
+        sw[tid * STR + LSQ] = f2_pack(wn, wn);
+    }
+    __syncthreads();
+    const uint64_t i0 = (uint64_t)blockIdx.x * (kEncThreads * 2 * kEncPairs) + tid;
+    uint64_t s[kEncPairs][LSQ], pn[kEncPairs];
+    bool ok[2 * kEncPairs];
+#pragma unroll
+    for (int q = 0; q < kEncPairs; ++q) {
+        float r[2][LSQ], n2[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint64_t i = i0 + (uint64_t)(2 * q + h) * kEncThreads;
+            bool in = i < p.n;
+            const uint32_t cell = in ? p.cell_assign[i] : 0u;
+            if ((uint64_t)cell >= (uint64_t)p.C * p.F) {
+                atomicExch(p.err, 1);
+                in = false;
+            }
+            ok[2 * q + h] = in;
+            const uint32_t c = cell / p.F, f = cell % p.F;
+#pragma unroll
+            for (int t = 0; t < LSQ; ++t)
+                r[h][t] = in ? residual<SECOND>(p, i, c, f, k * LSQ + t) : 0.0f;
+            n2[h] = pgpu::dot_seq(r[h], r[h], LSQ);
+        }
+#pragma unroll
+        for (int t = 0; t < LSQ; ++t) s[q][t] = f2_pack(r[0][t], r[1][t]);
+        pn[q] = f2_pack(n2[0], n2[1]);
+    }
+    float best[2 * kEncPairs];
+    int grp[2 * kEncPairs];
+#pragma unroll
+    for (int j = 0; j < 2 * kEncPairs; ++j) {
+        best[j] = FLT_MAX;
+        grp[j] = -1;
+    }
+    const uint64_t minus2 = f2_pack(-2.0f, -2.0f), one = f2_pack(p.one, p.one);
+#pragma unroll 1
+    for (int g = 0; g < 32; ++g) {
+        float gm[2 * kEncPairs];
+#pragma unroll
+        for (int j = 0; j < 2 * kEncPairs; ++j) gm[j] = FLT_MAX;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            uint64_t w[STR];
+#pragma unroll
+            for (int t = 0; t < STR; t += 2) {
+                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(&sw[(g * 8 + u) * STR + t]);
+                w[t] = v.x;
+                w[t + 1] = v.y;
+            }
+#pragma unroll
+            for (int q = 0; q < kEncPairs; ++q) {
+                uint64_t dt = f2_mul(s[q][0], w[0]);
+#pragma unroll
+                for (int t = 1; t < LSQ; ++t) dt = f2_fma(f2_mul(s[q][t], w[t]), one, dt);
+                float a, b;
+                f2_unpack(f2_fma(dt, minus2, f2_add(pn[q], w[LSQ])), a, b);
+                gm[2 * q] = fminf(gm[2 * q], a);
+                gm[2 * q + 1] = fminf(gm[2 * q + 1], b);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 2 * kEncPairs; ++j)
+            if (gm[j] < best[j]) {
+                best[j] = gm[j];
+                grp[j] = g;
+            }
+    }
+#pragma unroll
+    for (int j = 0; j < 2 * kEncPairs; ++j) {
+        if (!ok[j]) continue;
+        uint32_t bi = 0;
+        if (grp[j] >= 0) {
+            for (int u = 7; u >= 0; --u) {  // the last match found is the first in order
+                const uint64_t* w = &sw[(grp[j] * 8 + u) * STR];
+                uint64_t dt = f2_mul(s[j / 2][0], w[0]);
+#pragma unroll
+                for (int t = 1; t < LSQ; ++t) dt = f2_fma(f2_mul(s[j / 2][t], w[t]), one, dt);
+                float a, b;
+                f2_unpack(f2_fma(dt, minus2, f2_add(pn[j / 2], w[LSQ])), a, b);
+                if (((j & 1) ? b : a) == best[j]) bi = grp[j] * 8 + u;
+            }
+        }
+        const uint64_t i = i0 + (uint64_t)j * kEncThreads;
+        if (SECOND) p.p_codes[i * p.pnsq + k] = (uint8_t)bi;
+        else p.f_codes[i * p.fnsq + k] = (uint8_t)bi;
+    }
+}
+
+// One-dimensional codewords of each subspace in ascending order (value, then index), their
+// indexes, and whether any is too large (or not a number) for the search below.
+__global__ __launch_bounds__(256) void k_sort_levels(const float* __restrict__ cb,
+                                                     float* __restrict__ val, uint8_t* __restrict__ idx,
+                                                     int* __restrict__ bad) {
+    __shared__ float w[256];
+    const int tid = threadIdx.x;
+    const float x = cb[(uint64_t)blockIdx.x * 256 + tid];
+    w[tid] = x;
+    const int any = __syncthreads_or(!(fabsf(x) <= 1e18f));
+    int rank = 0;
+    for (int j = 0; j < 256; ++j) rank += (w[j] < x || (w[j] == x && j < tid)) ? 1 : 0;
+    if (tid == 0) bad[blockIdx.x] = any;
+    if (!any) {
+        val[(uint64_t)blockIdx.x * 256 + rank] = x;
+        idx[(uint64_t)blockIdx.x * 256 + rank] = (uint8_t)tid;
+    }
+}
+
+// The second quantizer over one-dimensional subspaces. The reference takes the smallest
+// cur_c = fl(fl(s^2 + w^2) - 2 fl(s w)), lowest index first; with u = 2^-24 each rounding is
+// within u of its operands' size, |cur_c - (s - w)^2| <= 8 u (s^2 + w^2). So no codeword is
+// the smallest whose (s - w)^2 less 16 u (s^2 + w^2) lies above a cur already found (twice
+// the bound: the test is in floats too), and once |s - w| > 2^-18 |w| that difference only
+// grows away from s: the scan from s's place in the sorted codewords stops there on each
+// side, after two or three codewords in practice. A warp takes a point's 32 dimensions,
+// block tiles of 32 dimensions keep the sorted codewords in shared memory (pitch 257: the
+// first steps of the 32 searches read 32 banks). @ENCODE1D@
+constexpr int k1dThreads = 512;
+constexpr int k1dPitch = 257;
+__global__ __launch_bounds__(k1dThreads) void k_encode_1d(AssignParams p, const float* __restrict__ val,
+                                                          const uint8_t* __restrict__ idx,
+                                                          const int* __restrict__ bad) {
+    __shared__ float sv[32 * k1dPitch];
+    __shared__ uint8_t si[32 * k1dPitch];
+    const int tid = threadIdx.x, lane = tid & 31;
+    const uint32_t t0 = blockIdx.y * 32, nt = p.d - t0 < 32 ? p.d - t0 : 32;
+    for (uint32_t e = tid; e < nt * 256; e += k1dThreads) {
+        sv[(e >> 8) * k1dPitch + (e & 255)] = val[(uint64_t)t0 * 256 + e];
+        si[(e >> 8) * k1dPitch + (e & 255)] = idx[(uint64_t)t0 * 256 + e];
+    }
+    __syncthreads();
+    const uint32_t t = t0 + lane;
+    const bool mine = (uint32_t)lane < nt;
+    const bool slow = mine && bad[t] != 0;
+    const float* w = sv + lane * k1dPitch;
+    const uint8_t* wi = si + lane * k1dPitch;
+    constexpr float kRel = 9.5367431640625e-07f;   // 2^-20 = 16 u
+    constexpr float kFar = 3.814697265625e-06f;    // 2^-18
+    constexpr float kTiny = 1e-36f;                // roundings of products below the normal range
+    const uint64_t step = (uint64_t)gridDim.x * (k1dThreads / 32);
+    for (uint64_t i = (uint64_t)blockIdx.x * (k1dThreads / 32) + (tid >> 5); i < p.n; i += step) {
+        const uint32_t cell = p.cell_assign[i];
+        if ((uint64_t)cell >= (uint64_t)p.C * p.F || !mine) continue;  // flagged by k_encode
+        const float s = residual<true>(p, i, cell / p.F, cell % p.F, t);
+        const float pn = __fmul_rn(s, s);
+        float best = FLT_MAX;
+        uint32_t bi = 0;
+        if (slow || !(fabsf(s) <= 1e18f)) {
+            for (uint32_t c = 0; c < 256; ++c) {
+                const float y = __ldg(p.pcb + (uint64_t)t * 256 + c);
+                const float cur = __fsub_rn(__fadd_rn(pn, __fmul_rn(y, y)), 2.0f * __fmul_rn(s, y));
+                if (cur < best) {
+                    best = cur;
+                    bi = c;
+                }
+            }
+        } else {
+            uint32_t pos = 0;  // codewords below s, at most 255
+#pragma unroll
+            for (int b = 128; b > 0; b >>= 1)
+                if (w[pos + b - 1] < s) pos += b;
+            bi = 256;
+            auto take = [&](int j) {  // false: no codeword further out can be the smallest
+                const float y = w[j];
+                const float yn = __fmul_rn(y, y), dd = fabsf(s - y);
+                if (dd > kFar * fabsf(y) && dd * dd - kRel * (dd * dd + pn + yn) - kTiny > best)
+                    return false;
+                const float cur = __fsub_rn(__fadd_rn(pn, yn), 2.0f * __fmul_rn(s, y));
+                const uint32_t c = wi[j];
+                if (cur < best || (cur == best && c < bi)) {
+                    best = cur;
+                    bi = c;
+                }
+                return true;
+            };
+            for (int j = (int)pos; j < 256; ++j)
+                if (!take(j)) break;
+            for (int j = (int)pos - 1; j >= 0; --j)
+                if (!take(j)) break;
+        }
+        p.p_codes[i * p.pnsq + t] = (uint8_t)bi;
+    }
+}
+
+// The offsets of a point, one thread each: 2 * sum_t decode(codes)[t] * vocab[t] with vocab =
+// coarse + fine, and for the second quantizer its decode against vocab + filter decode, the
+// sums sequential in t.
+__global__ __launch_bounds__(128) void k_offsets(AssignParams p, int vec) {
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= p.n) return;
+    const uint32_t cell = p.cell_assign[i];
+    if ((uint64_t)cell >= (uint64_t)p.C * p.F) return;
+    const float* cv = p.coarse + (uint64_t)(cell / p.F) * p.d;
+    const float* fv = p.fine + (uint64_t)(cell % p.F) * p.d;
+    const uint8_t* fc = p.f_codes + i * p.fnsq;
+    const uint8_t* pc = p.p_codes + i * p.pnsq;
+    float a = 0.0f, b = 0.0f;
+    if (vec) {
+        // four dimensions per step: d % 4 == 0, four-dimensional filter subspaces,
+        // 16-byte aligned centroids and codewords, one-dimensional second subspaces
+        for (uint32_t t = 0; t < p.d; t += 4) {
+            const float4 c4 = __ldg(reinterpret_cast<const float4*>(cv + t));
+            const float4 f4 = __ldg(reinterpret_cast<const float4*>(fv + t));
+            const float4 w4 = __ldg(reinterpret_cast<const float4*>(p.fcb) +
+                                    (uint64_t)(t >> 2) * 256 + fc[t >> 2]);
+            const float v[4] = {__fadd_rn(c4.x, f4.x), __fadd_rn(c4.y, f4.y), __fadd_rn(c4.z, f4.z),
+                                __fadd_rn(c4.w, f4.w)};
+            const float w[4] = {w4.x, w4.y, w4.z, w4.w};
+            float y[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                y[u] = p.pnsq ? __ldg(p.pcb + (uint64_t)(t + u) * 256 + pc[t + u]) : 0.0f;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                a = __fadd_rn(a, __fmul_rn(w[u], v[u]));
+                b = __fadd_rn(b, __fmul_rn(y[u], __fadd_rn(v[u], w[u])));
+            }
+        }
+    } else {
+        for (uint32_t t = 0; t < p.d; ++t) {
+            const float v = __fadd_rn(__ldg(cv + t), __ldg(fv + t));
+            const uint32_t k = t / p.flsq;
+            const float w = __ldg(p.fcb + ((uint64_t)k * 256 + fc[k]) * p.flsq + (t - k * p.flsq));
+            a = __fadd_rn(a, __fmul_rn(w, v));
+            if (p.pnsq) {
+                const uint32_t m = t / p.plsq;
+                const float y = __ldg(p.pcb + ((uint64_t)m * 256 + pc[m]) * p.plsq + (t - m * p.plsq));
+                b = __fadd_rn(b, __fmul_rn(y, __fadd_rn(v, w)));
+            }
+        }
+    }
+    p.f_off[i] = 2.0f * a;
+    if (p.pnsq) p.p_off[i] = 2.0f * b;
+}
+
+template <bool SECOND>
+void launch_encode(const AssignParams& p, uint32_t nsq, uint32_t lsq, cudaStream_t st) {
+    constexpr uint32_t per = kEncThreads * 2 * kEncPairs;
+    const dim3 grid((unsigned)((p.n + per - 1) / per), nsq);
+    switch (lsq) {
+#define PGPU_ENC(L) \
+    case L:         \
+        k_encode<L, SECOND><<<grid, kEncThreads, 0, st>>>(p); \
+        break;
+        PGPU_ENC(1) PGPU_ENC(2) PGPU_ENC(3) PGPU_ENC(4) PGPU_ENC(5) PGPU_ENC(6) PGPU_ENC(7) PGPU_ENC(8)
+#undef PGPU_ENC
+    }
+}
+
 }  // namespace
 
 extern "C" int pgpu_puck_assign(uint32_t d, uint64_t n, const float* base,
@@ -181,13 +506,20 @@ extern "C" int pgpu_puck_assign(uint32_t d, uint64_t n, const float* base,
     p.flsq = d / filter_nsq;
     p.pnsq = pq_nsq;
     p.plsq = pq_nsq ? d / pq_nsq : 0;
+    p.one = 1.0f;
     // residual and vocab floats, then the two code rows, rounded up to whole floats
     p.stride = 2 * d + (filter_nsq + pq_nsq + 3) / 4;
     const size_t smem = sizeof(float) * kAssignWarps * p.stride;  // <= 72 KB (d <= kMaxDim)
     const uint64_t nnorm = (uint64_t)(filter_nsq + pq_nsq) * 256;
+    // subspaces of at most 8 dimensions (every shape of the configurations): the kernels
+    // that are parallel over subspaces; @RULE@
+    const bool split = p.flsq <= 8 && p.plsq <= 8;
+    const bool sorted = split && pq_nsq && p.plsq == 1;
     float* norms = nullptr;
     int* err = nullptr;
-    cudaError_t e = cudaMallocAsync((void**)&norms, sizeof(float) * nnorm + sizeof(int), st);
+    cudaError_t e = cudaMallocAsync(
+        (void**)&norms,
+        sizeof(float) * nnorm + sizeof(int) + (sorted ? d * (256ull * 5 + sizeof(int)) : 0), st);
     if (e != cudaSuccess)
         return pgpu::set_last_error(e == cudaErrorMemoryAllocation ? PGPU_E_NOMEM : PGPU_E_CUDA,
                                     std::string("puck_assign scratch: ") + cudaGetErrorString(e));
@@ -203,8 +535,27 @@ extern "C" int pgpu_puck_assign(uint32_t d, uint64_t n, const float* base,
         if (pq_nsq)
             k_codeword_norms<<<(unsigned)((pq_nsq * 256ull + 255) / 256), 256, 0, st>>>(
                 pq_codebook, pq_nsq * 256ull, p.plsq, norms + (uint64_t)filter_nsq * 256);
-        k_puck_assign<<<(unsigned)((n + kAssignWarps - 1) / kAssignWarps), kAssignWarps * 32, smem,
-                        st>>>(p);
+        if (split) {
+            launch_encode<false>(p, filter_nsq, p.flsq, st);
+            if (sorted) {
+                int* bad = err + 1;
+                float* val = reinterpret_cast<float*>(bad + d);
+                uint8_t* idx = reinterpret_cast<uint8_t*>(val + (uint64_t)d * 256);
+                k_sort_levels<<<d, 256, 0, st>>>(pq_codebook, val, idx, bad);
+                const uint64_t want = (n + k1dThreads / 32 - 1) / (k1dThreads / 32);
+                const dim3 grid((unsigned)(want < 2048 ? want : 2048), (d + 31) / 32);
+                k_encode_1d<<<grid, k1dThreads, 0, st>>>(p, val, idx, bad);
+            } else if (pq_nsq) {
+                launch_encode<true>(p, pq_nsq, p.plsq, st);
+            }
+            const auto aligned = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+            const int vec = p.flsq == 4 && p.plsq <= 1 && aligned(coarse) && aligned(fine) &&
+                            aligned(filter_codebook);
+            k_offsets<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(p, vec);
+        } else {
+            k_puck_assign<<<(unsigned)((n + kAssignWarps - 1) / kAssignWarps), kAssignWarps * 32, smem,
+                            st>>>(p);
+        }
         e = cudaGetLastError();
     }
     int flag = 0;

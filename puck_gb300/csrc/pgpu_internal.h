@@ -331,6 +331,8 @@ struct TcEpilogue {
     float* out2;
     float alpha, beta;
 };
+// SMs of the calling thread's current device.
+int sm_count();
 size_t tc_gemm_smem_bytes();
 cudaError_t launch_tc_gemm(const TcOperand& A, const TcOperand& B, uint32_t K,
                            const TcEpilogue& ep, int* err, cudaStream_t stream);

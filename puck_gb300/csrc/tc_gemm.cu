@@ -704,17 +704,6 @@ bool encode_operand(CUtensorMap* map, const TcOperand& op, uint32_t K, uint32_t 
               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-int sm_count() {
-    static std::mutex mu;
-    static int counts[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    std::lock_guard<std::mutex> g(mu);
-    if (dev >= 0 && dev < 64 && counts[dev] == 0)
-        cudaDeviceGetAttribute(&counts[dev], cudaDevAttrMultiProcessorCount, dev);
-    return dev >= 0 && dev < 64 && counts[dev] > 0 ? counts[dev] : 1;
-}
-
 // The persistent TMA form applies: both operands BF16, rows 16-byte aligned, every
 // row read in place (no gather, no device row count).
 bool tma_applies(const TcOperand& A, const TcOperand& B, uint32_t K) {
@@ -768,6 +757,17 @@ cudaError_t launch_tc_gemm_tma(const TcOperand& A, const TcOperand& B, uint32_t 
 }
 
 }  // namespace
+
+int sm_count() {
+    static std::mutex mu;
+    static int counts[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> g(mu);
+    if (dev >= 0 && dev < 64 && counts[dev] == 0)
+        cudaDeviceGetAttribute(&counts[dev], cudaDevAttrMultiProcessorCount, dev);
+    return dev >= 0 && dev < 64 && counts[dev] > 0 ? counts[dev] : 1;
+}
 
 size_t tc_gemm_smem_bytes() { return 2 * (size_t)kStageBytes; }
 size_t tc_gemm_async_smem_bytes() { return kAsyncStages * (size_t)kStageBytes; }

@@ -46,15 +46,22 @@ def test_walk_heap_shapes(indexes, name, T):
     path, q = indexes[name]
     k = min(T, 20)
     P = 1000  # clamped to the index's clusters: every one is probed
-    ix = native.GpuIndex(path, search_coarse_count=P, filter_topk=T, topk=k, max_batch=96)
+    # the same queries as one pass of 192 blocks (more than SMs) and two of 96
+    ix = native.GpuIndex(path, search_coarse_count=P, filter_topk=T, topk=k, max_batch=192)
+    wide, wide_ids = ix.search(np.concatenate([q, q]), k)
+    assert np.array_equal(_bits(wide[:96]), _bits(wide[96:])) and np.array_equal(wide_ids[:96], wide_ids[96:])
     dist, ids = ix.search(q, k)
     stats = ix.last_stats()
+    assert np.array_equal(_bits(dist), _bits(wide[:96])) and np.array_equal(ids, wide_ids[:96])
     ix.close()
-    od, oi, st = oracle.OracleIndex(path).search_batch(q, k, P, T, topk_max=k, nthreads=os.cpu_count())
+    orc = oracle.OracleIndex(path)
+    od, oi, st = orc.search_batch(q, k, P, T, topk_max=k, nthreads=os.cpu_count())
     assert (st == 0).all()
     assert np.array_equal(_bits(dist), _bits(od))
     assert np.array_equal(ids, oi)
-    assert stats["records_scanned"] >= min(T, 12000)
+    traces = [orc.search_one(x, k, P, T, topk_max=k, trace=True)[4] for x in q]
+    assert stats["cells_scanned"] == sum(t["scanned_cells"] for t in traces)
+    assert stats["records_scanned"] == sum(t["scanned_points"] for t in traces)
 
 
 @pytest.mark.parametrize("rate", [1.0, 1.3])

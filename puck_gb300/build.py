@@ -34,7 +34,7 @@ def _needs_rebuild():
     if not os.path.exists(LIB):
         return True
     t = os.path.getmtime(LIB)
-    deps = sources() + [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".h")]
+    deps = sources() + [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh"))]
     deps.append(os.path.join(os.path.dirname(HERE), "include", "puck_gb300.h"))
     return any(os.path.getmtime(p) > t for p in deps)
 

@@ -336,6 +336,31 @@ int sm_count();
 size_t tc_gemm_smem_bytes();
 cudaError_t launch_tc_gemm(const TcOperand& A, const TcOperand& B, uint32_t K,
                            const TcEpilogue& ep, int* err, cudaStream_t stream);
+// Contraction with a selecting epilogue (tc_filter.cu): s_ij = bias_j - a_i.b_j over BF16 rows.
+constexpr uint32_t kTcFilterTile = 256;  // columns per tile
+enum { kTcMinima = 0, kTcBelow = 1, kTcDense = 2 };
+struct TcFilter {
+    uint32_t M, N, K;          // rows of A and B, dimensions (tc_filter_applies)
+    const float* bias;         // [tiles * kTcFilterTile], FLT_MAX past N
+    uint32_t pos0, pos1;       // positions [pos0, pos1): tile (position * step) mod tiles
+    uint32_t step, tiles;
+    float* gmin;               // MINIMA: [M][tiles * 32] smallest score per 8 columns
+    const float* thr;          // BELOW: [M] thresholds
+    uint32_t* count;           // BELOW: [M] list lengths so far (beyond cap: entries lost)
+    uint2* cand;               // BELOW, DENSE: [M][cap] (score bits, id0 + column)
+    uint32_t cap, id0;
+    int* err;
+    uint32_t splits;           // set by the launcher
+};
+bool tc_filter_applies(uint32_t K);
+cudaError_t launch_tc_filter(int mode, const uint16_t* A, uint64_t a_rs, const uint16_t* B,
+                             uint64_t b_rs, TcFilter p, cudaStream_t stream);
+// BF16 copies of rows, dp values apart, and |x|^2 (seq: products and sums rounded separately)
+// or 0.5|x|^2 (fused, `pad` entries of FLT_MAX after the rows); lost (optional): a bound on
+// |x - bf16(x)|.
+cudaError_t launch_rows_bf16(const float* X, uint64_t rows, uint32_t d, uint32_t dp, bool seq,
+                             uint32_t pad, uint16_t* out, float* norm, float* lost,
+                             cudaStream_t stream);
 // Exact selections over a tensor-core screen (tc_select.cu).
 size_t window_smem_bytes(uint32_t C, uint32_t d);
 cudaError_t launch_abs_from_half_norms(const float* half_norms, uint32_t n, float* out,

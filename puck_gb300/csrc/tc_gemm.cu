@@ -24,6 +24,7 @@
 #include <mutex>
 
 #include "pgpu_internal.h"
+#include "tc_common.cuh"
 
 namespace pgpu {
 namespace {
@@ -33,10 +34,6 @@ constexpr uint32_t kTileM = 128, kTileN = 128, kChunkK = 64;
 constexpr uint32_t kTmemCols = 128;
 constexpr uint32_t kStageBytes = (kTileM + kTileN) * kChunkK * 2;  // 32 KiB
 constexpr uint32_t kWaitLimit = 1u << 22;
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-    return (uint32_t)__cvta_generic_to_shared(p);
-}
 
 // Shared-memory matrix descriptor: start address, leading byte offset (between
 // core matrices along K), stride byte offset (between 8-row groups), the fixed
@@ -430,29 +427,6 @@ __host__ __device__ constexpr uint32_t tma_stage_bytes(int nt) {
     return kTmaABytes + (uint32_t)nt * kTmaK * 2u;
 }
 
-// K-major, 128-byte swizzled operand tile (8-row x 128-byte atoms, 1024 bytes apart):
-// start address, leading byte offset 16 (unused within one atom), stride byte offset
-// 1024, the fixed 0b001 at bits 46-48, swizzle mode 2 (128 B) at bits 61-63.
-__device__ __forceinline__ uint64_t sw128_desc(uint32_t addr) {
-    return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)1u << 16) |
-           ((uint64_t)(1024u >> 4) << 32) | (1ull << 46) | (2ull << 61);
-}
-
-__device__ __forceinline__ bool tma_wait(uint32_t bar, uint32_t parity, const volatile int* failed) {
-    for (uint32_t it = 0; it < kWaitLimit; ++it) {
-        uint32_t ok;
-        asm volatile(
-            "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-            "selp.b32 %0, 1, 0, p;\n}"
-            : "=r"(ok)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (ok) return true;
-        if ((it & 1023u) == 1023u && *failed) return false;
-    }
-    return false;
-}
-
 template <int EPI, int NT>
 __global__ __launch_bounds__(kTmaThreads, 1) void k_tc_gemm_tma(
     const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
@@ -664,12 +638,6 @@ __global__ __launch_bounds__(kTmaThreads, 1) void k_tc_gemm_tma(
     }
 }
 
-bool operand_vec(const TcOperand& op) {
-    if (op.pb != nullptr)
-        return op.ks == 1 && (op.rs & 7u) == 0 && (reinterpret_cast<uintptr_t>(op.pb) & 15u) == 0;
-    return op.ks == 1 && (op.rs & 3u) == 0 && (reinterpret_cast<uintptr_t>(op.p) & 15u) == 0;
-}
-
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link to the
 // driver library).
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
@@ -690,18 +658,10 @@ EncodeTiledFn encode_tiled_fn() {
     return fn;
 }
 
-// 2-D BF16 tensor map of an operand (rows x K, row stride rs elements), box 64 (K)
-// x box_rows, 128-byte swizzle, zero fill past the ends.
-bool encode_operand(CUtensorMap* map, const TcOperand& op, uint32_t K, uint32_t box_rows) {
-    EncodeTiledFn fn = encode_tiled_fn();
-    if (fn == nullptr) return false;
-    const cuuint64_t dims[2] = {K, op.rows};
-    const cuuint64_t strides[1] = {op.rs * 2ull};
-    const cuuint32_t box[2] = {kTmaK, box_rows};
-    const cuuint32_t estr[2] = {1, 1};
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<uint16_t*>(op.pb), dims, strides,
-              box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+bool operand_vec(const TcOperand& op) {
+    if (op.pb != nullptr)
+        return op.ks == 1 && (op.rs & 7u) == 0 && (reinterpret_cast<uintptr_t>(op.pb) & 15u) == 0;
+    return op.ks == 1 && (op.rs & 3u) == 0 && (reinterpret_cast<uintptr_t>(op.p) & 15u) == 0;
 }
 
 // The persistent TMA form applies: both operands BF16, rows 16-byte aligned, every
@@ -723,7 +683,8 @@ cudaError_t launch_tc_gemm_tma(const TcOperand& A, const TcOperand& B, uint32_t 
                        ? 256
                        : 128;
     CUtensorMap ma, mb;
-    if (!encode_operand(&ma, A, K, 128) || !encode_operand(&mb, B, K, (uint32_t)nt))
+    if (!encode_bf16_rows(&ma, A.pb, A.rows, A.rs, K, 128) ||
+        !encode_bf16_rows(&mb, B.pb, B.rows, B.rs, K, (uint32_t)nt))
         return cudaSuccess;  // not encodable: the cp.async form runs instead
     const uint64_t tiles = tiles_m * ((B.rows + nt - 1) / nt);
     const unsigned grid = (unsigned)(tiles < (uint64_t)sm_count() ? tiles : (uint64_t)sm_count());
@@ -757,6 +718,19 @@ cudaError_t launch_tc_gemm_tma(const TcOperand& A, const TcOperand& B, uint32_t 
 }
 
 }  // namespace
+
+bool encode_bf16_rows(CUtensorMap* map, const uint16_t* p, uint64_t rows, uint64_t rs, uint32_t K,
+                      uint32_t box_rows) {
+    EncodeTiledFn fn = encode_tiled_fn();
+    if (fn == nullptr) return false;
+    const cuuint64_t dims[2] = {K, rows};
+    const cuuint64_t strides[1] = {rs * 2ull};
+    const cuuint32_t box[2] = {kTmaK, box_rows};
+    const cuuint32_t estr[2] = {1, 1};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<uint16_t*>(p), dims, strides, box,
+              estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
 
 int sm_count() {
     static std::mutex mu;

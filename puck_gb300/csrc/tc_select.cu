@@ -343,8 +343,167 @@ __global__ __launch_bounds__(256) void k_window_small(
     }
 }
 
-// nearest_center (kmeans.cpp:221-258) from a tensor-core screen: one warp per
-// point. s^_j ~ 0.5|c_j|^2 - x.c_j orders the centroids like the reference's
+// nearest_center, exact part after the MINIMA screen (tc_filter.cu): one warp per point. With
+// xa = |x|, dx = |x - bf16(x)| and cmax, dcmax the largest |c| and |c - bf16(c)|, every
+// screened score is within
+//   E = dx cmax + (xa + dx) dcmax + (d + 8) 2^-21 (xa + dx)(cmax + dcmax)
+//       + 2^-21 (xn + cmax^2) + 2^-20 (0.5 cmax^2 + 1.01 xa cmax)
+// of the value that orders the centroids like the reference's cur_j = (|x|^2 + |c_j|^2) -
+// 2 x.c_j (the roundings of the operands, of both accumulations, of the final subtractions), so
+// the centroid with the smallest cur_j, and every one equal to it, lies in a group of 8 whose
+// smallest score is at most the row's smallest + 2E. Those groups (1.3 per point where the
+// clusters are apart) are measured in the reference's FP32 order, lane = centroid; the smallest
+// cur_j with the lowest id wins, as in the reference's strict-< scan. Rows or centroids too
+// large for the bound, or a failed screen: every group. Eight lanes per point, four points per
+// warp; bound by the L2 and L1 traffic of the centroid rows, for which groups of 8 are read by
+// the row (groups of 32 read as columns of a transposed copy took 135 us for 77824 points of 96
+// dimensions against 2000 centroids, groups of 8 so 160, this 90). The whole call on 262144 such
+// points: 3.57 ms with a screen matrix in memory, 0.60 now; 131072 points of 4 dimensions
+// against 256 codewords 184 us, now 90.
+constexpr int kArgminWarps = 8;
+constexpr int kArgminRows = kArgminWarps * 4;  // points per block
+struct CentsMax {
+    uint32_t norm2_bits;  // largest |c|^2
+    uint32_t lost_bits;   // largest |c - bf16(c)|
+};
+__global__ __launch_bounds__(kArgminWarps * 32) void k_group_argmin(
+    const float* __restrict__ gmin, uint32_t G, const float* __restrict__ X, uint64_t row0,
+    uint32_t rows, uint32_t d, const float* __restrict__ xnorm, const float* __restrict__ xlost,
+    const float* __restrict__ cents, const float* __restrict__ cnorm,
+    const CentsMax* __restrict__ cmax, uint32_t K, int vec, const int* __restrict__ tc_err,
+    int32_t* __restrict__ assign, float* __restrict__ dis) {
+    extern __shared__ __align__(16) float argmin_rows[];  // [kArgminRows][pitch]
+    const int lane = threadIdx.x & 31, l8 = lane & 7;
+    const uint32_t slot = threadIdx.x >> 3, w = blockIdx.x * kArgminRows + slot;
+    const bool valid = w < rows;
+    const uint64_t p = row0 + (valid ? w : 0u);
+    const uint32_t pitch = ((d + 3u) & ~3u) + 4u;  // the four points of a warp in other banks
+    float* x = argmin_rows + (uint64_t)slot * pitch;
+    for (uint32_t t = l8; t < d; t += 8) x[t] = X[p * d + t];
+    // the row's minima, 256 at a time (32 per lane): one read up to 2048 centroids
+    const float4* gm = reinterpret_cast<const float4*>(gmin + (uint64_t)(valid ? w : 0u) * G);
+    float4 v[8];
+    auto fetch = [&](uint32_t i0) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const uint32_t i = i0 + 8 * u + l8;
+            v[u] = i < G / 4 ? gm[i] : make_float4(FLT_MAX, FLT_MAX, FLT_MAX, FLT_MAX);
+        }
+    };
+    float U = FLT_MAX;
+    for (uint32_t i0 = 0; i0 < G / 4; i0 += 64) {
+        fetch(i0);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) U = fminf(U, fminf(fminf(v[u].x, v[u].y), fminf(v[u].z, v[u].w)));
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) U = fminf(U, __shfl_xor_sync(0xffffffffu, U, o));
+    const float xn = xnorm[valid ? w : 0u], xa = sqrtf(xn), dx = xlost[valid ? w : 0u];
+    const float c2 = __uint_as_float(cmax->norm2_bits), ca = sqrtf(c2) * 1.0000005f;
+    const float dc = __uint_as_float(cmax->lost_bits);
+    const float E = dx * ca + (xa + dx) * dc +
+                    (float)(d + 8) * 4.76837158203125e-07f * (xa + dx) * (ca + dc) +
+                    4.76837158203125e-07f * (xn + c2) +
+                    9.5367431640625e-07f * (0.5f * c2 + 1.01f * xa * ca) + 1e-30f;
+    const bool all = *tc_err != 0 || !(xn < 1e36f) || !(c2 < 1e36f);
+    const float thr = U + 2.0f * E * 1.00001f;
+    __syncwarp();
+    // the reference's scan: min starts at FLT_MAX, strict < in ascending id order (a value of
+    // FLT_MAX is none: bidx 0 keeps it out)
+    float best = FLT_MAX;
+    uint32_t bidx = 0;
+    const uint32_t groups = (K + 7) / 8;
+    for (uint32_t i0 = 0; i0 < G / 4; i0 += 64) {
+        if (G > 256) fetch(i0);
+        uint32_t mask = 0;  // bit 4u + e: this lane's group 4 (i0 + 8u + l8) + e
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            mask |= ((all || v[u].x <= thr ? 1u : 0u) | (all || v[u].y <= thr ? 2u : 0u) |
+                     (all || v[u].z <= thr ? 4u : 0u) | (all || v[u].w <= thr ? 8u : 0u)) << (4 * u);
+        if (!valid) mask = 0;
+        for (;;) {
+            const unsigned left = __ballot_sync(0xffffffffu, mask != 0);
+            if (left == 0) break;
+            const unsigned team = (left >> (lane & 24)) & 255u;
+            const int src = team ? __ffs(team) - 1 : 0;  // a lane of the point with a group
+            const uint32_t theirs = __shfl_sync(0xffffffffu, mask, (lane & 24) + src);
+            if (team == 0) continue;  // another point of the warp has one
+            if (l8 == src) mask &= mask - 1;
+            const uint32_t bit = __ffs(theirs) - 1;
+            const uint32_t g = (i0 + 8 * (bit >> 2) + src) * 4 + (bit & 3), j = g * 8 + l8;
+            if (g >= groups || j >= K) continue;
+            const float* cj = cents + (uint64_t)j * d;
+            float s = 0.0f;
+            if (vec) {
+                // 32 bytes per load: each of a warp's loads reads 32 rows, a line each
+#pragma unroll 4
+                for (uint32_t t = 0; t < d; t += 8) {
+                    float y[8];
+                    asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                        : "=f"(y[0]), "=f"(y[1]), "=f"(y[2]), "=f"(y[3]), "=f"(y[4]), "=f"(y[5]),
+                          "=f"(y[6]), "=f"(y[7])
+                        : "l"(cj + t));
+                    const float4 q0 = *reinterpret_cast<const float4*>(x + t);
+                    const float4 q1 = *reinterpret_cast<const float4*>(x + t + 4);
+                    s = __fadd_rn(s, __fmul_rn(q0.x, y[0]));
+                    s = __fadd_rn(s, __fmul_rn(q0.y, y[1]));
+                    s = __fadd_rn(s, __fmul_rn(q0.z, y[2]));
+                    s = __fadd_rn(s, __fmul_rn(q0.w, y[3]));
+                    s = __fadd_rn(s, __fmul_rn(q1.x, y[4]));
+                    s = __fadd_rn(s, __fmul_rn(q1.y, y[5]));
+                    s = __fadd_rn(s, __fmul_rn(q1.z, y[6]));
+                    s = __fadd_rn(s, __fmul_rn(q1.w, y[7]));
+                }
+            } else if (d == 4 && (reinterpret_cast<uintptr_t>(cents) & 15) == 0) {
+                const float4 y = __ldg(reinterpret_cast<const float4*>(cj));
+                s = __fadd_rn(s, __fmul_rn(x[0], y.x));
+                s = __fadd_rn(s, __fmul_rn(x[1], y.y));
+                s = __fadd_rn(s, __fmul_rn(x[2], y.z));
+                s = __fadd_rn(s, __fmul_rn(x[3], y.w));
+            } else {
+                for (uint32_t t = 0; t < d; ++t) s = __fadd_rn(s, __fmul_rn(x[t], __ldg(cj + t)));
+            }
+            const float cur = __fsub_rn(__fadd_rn(xn, cnorm[j]), 2.0f * s);
+            if (cur < best || (cur == best && j < bidx)) {
+                best = cur;
+                bidx = j;
+            }
+        }
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, best, o);
+        const uint32_t oi = __shfl_xor_sync(0xffffffffu, bidx, o);
+        if (ov < best || (ov == best && oi < bidx)) {
+            best = ov;
+            bidx = oi;
+        }
+    }
+    if (valid && l8 == 0) {
+        assign[p] = (int32_t)bidx;
+        dis[p] = best;
+    }
+}
+
+// The screen's bias 0.5|c|^2 (FLT_MAX past the centroids), and the largest norm and rounding
+// loss (their bits: the order of non-negative floats; no number is above all).
+__global__ void k_cents_bias(const float* __restrict__ cnorm, const float* __restrict__ clost,
+                             uint32_t K, uint32_t n, float* __restrict__ bias,
+                             CentsMax* __restrict__ cmax) {
+    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;  // n: whole blocks
+    const float c = j < K ? cnorm[j] : 0.0f, l = j < K ? clost[j] : 0.0f;
+    if (j < n) bias[j] = j < K ? 0.5f * c : FLT_MAX;
+    const uint32_t mc = __reduce_max_sync(0xffffffffu, __float_as_uint(c));
+    const uint32_t ml = __reduce_max_sync(0xffffffffu, __float_as_uint(l));
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(&cmax->norm2_bits, mc);
+        atomicMax(&cmax->lost_bits, ml);
+    }
+}
+
+// nearest_center without the selecting screen (dimensions above its limit): one warp per
+// point over the whole screen matrix.
+// s^_j ~ 0.5|c_j|^2 - x.c_j orders the centroids like the reference's
 // cur_j = (|x|^2 + |c_j|^2) - 2 x.c_j; the window around the screened minimum
 // is recomputed exactly and the smallest cur_j with the lowest id wins, as in
 // the reference's strict-< scan.
@@ -475,9 +634,76 @@ cudaError_t launch_coarse_window(const DeviceIndex& ix, uint32_t n, Scratch& s,
     return cudaGetLastError();
 }
 
+// nearest_center through the MINIMA screen (k_tc_filter) and k_group_argmin, in chunks whose
+// BF16 rows and group minima stay in L2 between the kernels; a call allocates 50 MB at most
+// beside the centroids' copies.
+static cudaError_t nearest_center_screened(uint32_t dim, const float* cents, uint32_t k, const float* x,
+                                           uint64_t n, int32_t* assign, float* dis,
+                                           cudaStream_t stream) {
+    const uint32_t dp = (dim + 7u) & ~7u;
+    const uint32_t tiles = (k + kTcFilterTile - 1) / kTcFilterTile, kp = tiles * kTcFilterTile;
+    const uint32_t G = tiles * (kTcFilterTile / 8);
+    // whole waves of 128-row tiles (one per SM) within 48 MiB of row scratch
+    const uint64_t wave = 128ull * (uint64_t)sm_count();
+    uint64_t chunk = (48ull << 20) / (2ull * dp + 8 + 4ull * G);
+    chunk = chunk >= wave ? chunk / wave * wave : chunk >= 128 ? chunk / 128 * 128 : 128;
+    if (chunk > n) chunk = n;
+    // one allocation, 256-byte aligned parts
+    uint64_t bytes = 0;
+    auto part = [&](uint64_t size) {
+        const uint64_t at = bytes;
+        bytes += (size + 255) & ~255ull;
+        return at;
+    };
+    const uint64_t o_flags = part(sizeof(CentsMax) + 4), o_cb = part(2ull * k * dp), o_cn = part(4ull * k),
+                   o_cl = part(4ull * k), o_bias = part(4ull * kp),
+                   o_xb = part(2ull * chunk * dp), o_xn = part(4ull * chunk), o_xl = part(4ull * chunk),
+                   o_gm = part(4ull * chunk * G);
+    uint8_t* base = nullptr;
+    cudaError_t e = cudaMallocAsync((void**)&base, bytes, stream);
+    if (e != cudaSuccess) return e;
+    CentsMax* cmax = reinterpret_cast<CentsMax*>(base + o_flags);
+    int* err = reinterpret_cast<int*>(cmax + 1);
+    uint16_t* cb = reinterpret_cast<uint16_t*>(base + o_cb);
+    uint16_t* xb = reinterpret_cast<uint16_t*>(base + o_xb);
+    auto f = [&](uint64_t at) { return reinterpret_cast<float*>(base + at); };
+    e = cudaMemsetAsync(cmax, 0, sizeof(CentsMax) + 4, stream);
+    if (e == cudaSuccess)
+        e = launch_rows_bf16(cents, k, dim, dp, true, 0, cb, f(o_cn), f(o_cl), stream);
+    if (e == cudaSuccess) {
+        k_cents_bias<<<(kp + 255) / 256, 256, 0, stream>>>(f(o_cn), f(o_cl), k, kp, f(o_bias), cmax);
+        e = cudaGetLastError();
+    }
+    const size_t smem = sizeof(float) * kArgminRows * (((dim + 3u) & ~3u) + 4u);  // <= 33 KB
+    const int vec = dim % 8 == 0 && (reinterpret_cast<uintptr_t>(cents) & 31) == 0;
+    for (uint64_t r0 = 0; e == cudaSuccess && r0 < n; r0 += chunk) {
+        const uint32_t rows = (uint32_t)(n - r0 < chunk ? n - r0 : chunk);
+        e = launch_rows_bf16(x + r0 * dim, rows, dim, dp, true, 0, xb, f(o_xn), f(o_xl), stream);
+        TcFilter p{};
+        p.M = rows;
+        p.N = k;
+        p.K = dim;
+        p.bias = f(o_bias);
+        p.pos1 = p.tiles = tiles;
+        p.step = 1;
+        p.gmin = f(o_gm);
+        p.err = err;
+        if (e == cudaSuccess) e = launch_tc_filter(kTcMinima, xb, dp, cb, dp, p, stream);
+        if (e != cudaSuccess) break;
+        k_group_argmin<<<(rows + kArgminRows - 1) / kArgminRows, kArgminWarps * 32, smem, stream>>>(
+            f(o_gm), G, x, r0, rows, dim, f(o_xn), f(o_xl), cents, f(o_cn), cmax, k, vec, err, assign, dis);
+        e = cudaGetLastError();
+    }
+    cudaFreeAsync(base, stream);
+    return e;
+}
+
 cudaError_t launch_nearest_center_tc(uint32_t dim, const float* cents, uint64_t k, const float* x,
                                      uint64_t n, int32_t* assign, float* dis, cudaStream_t stream) {
     if (n == 0) return cudaSuccess;
+    // k below 2^24: the minima of a row stay below 8 MB
+    if (tc_filter_applies(dim) && k < (1ull << 24))
+        return nearest_center_screened(dim, cents, (uint32_t)k, x, n, assign, dis, stream);
     // screen buffer of at most 256 MiB: rows per chunk, a multiple of 128
     uint64_t chunk = (256ull << 20) / (4 * (k ? k : 1));
     chunk = chunk < 128 ? 128 : (chunk / 128) * 128;

@@ -346,15 +346,17 @@ struct TcFilter {
     uint32_t step, tiles;
     float* gmin;               // MINIMA: [M][tiles * 32] smallest score per 8 columns
     const float* thr;          // BELOW: [M] thresholds
-    uint32_t* count;           // BELOW: [M] list lengths so far (beyond cap: entries lost)
-    uint2* cand;               // BELOW, DENSE: [M][cap] (score bits, id0 + column)
+    uint32_t* count;           // BELOW: [M][2 splits] entries of each part (above seg: some lost)
+    uint2* cand;               // (score bits, id0 + column): BELOW [M][2 splits] parts of seg in
+                               // rows of cap, DENSE [M][cap] in the order of the positions
     uint32_t cap, id0;
     int* err;
-    uint32_t splits;           // set by the launcher
+    uint32_t splits, seg;      // set by the launcher: splits (tc_filter_splits at most), cap / (2 splits)
 };
+uint32_t tc_filter_splits(uint32_t M);
 bool tc_filter_applies(uint32_t K);
 cudaError_t launch_tc_filter(int mode, const uint16_t* A, uint64_t a_rs, const uint16_t* B,
-                             uint64_t b_rs, TcFilter p, cudaStream_t stream);
+                             uint64_t b_rs, TcFilter& p, cudaStream_t stream);
 // BF16 copies of rows, dp values apart, and |x|^2 (seq: products and sums rounded separately)
 // or 0.5|x|^2 (fused, `pad` entries of FLT_MAX after the rows); lost (optional): a bound on
 // |x - bf16(x)|.
@@ -391,8 +393,12 @@ cudaError_t launch_probe_select(const ProbeNet& net, const DeviceIndex& ix, uint
                                 cudaStream_t st);
 
 // Brute-force kNN on the tensor-core screen with FP32 rescoring (knn.cu); k <= 64.
+// flags (DEVICE): [0] a tensor-core wait expired, [1] a candidate list overflowed: the result
+// is not valid, launch_knn_dense gives it.
 cudaError_t launch_knn(const float* base, uint64_t n, uint32_t d, const float* Q, uint32_t nq,
-                       uint32_t k, uint32_t* ids, float* dist, int* err, cudaStream_t st);
+                       uint32_t k, uint32_t* ids, float* dist, int* flags, cudaStream_t st);
+cudaError_t launch_knn_dense(const float* base, uint64_t n, uint32_t d, const float* Q, uint32_t nq,
+                             uint32_t k, uint32_t* ids, float* dist, int* err, cudaStream_t st);
 const ProbeNet* probe_net(const pgpu_probe* p);
 int probe_device(const pgpu_probe* p);
 

@@ -5,8 +5,10 @@
 //           nearest_center. The centroid nearest to a point lies in a group whose minimum is
 //           within twice the screen's error of the row's smallest; only those groups are
 //           measured exactly.
-//   BELOW   the (score, column) pairs at or below a row's threshold, appended to its list: the
-//           screen of the brute-force neighbours. DENSE fills the lists for the first columns.
+//   BELOW   the (score, column) pairs at or below a row's threshold, in its list: the screen of
+//           the brute-force neighbours. A row's list has a part for each warp that works on the
+//           row, so an entry costs no atomic (one with its result on the way took 3 of the 6 ms
+//           of a million columns). DENSE fills the lists for the first columns.
 //
 // One CTA per SM loops over items, an item being a 128-row tile of A and every splits-th of a
 // range of 256-column tiles of B (position p stands for tile (p * step) mod tiles: a range of
@@ -212,16 +214,28 @@ __global__ __launch_bounds__(kThreads, 1) void k_tc_filter(const __grid_constant
             const uint32_t row = item / p.splits * 128u + quarter * 32u + lane;
             const bool in = row < p.M;
             const float thr = MODE == kTcBelow && in ? p.thr[row] : -FLT_MAX;
+            // this warp's part of the row's list: no other warp of the grid writes it
+            const uint32_t part = item % p.splits * 2 + half;
+            uint2* list = p.cand + (uint64_t)row * p.cap + part * p.seg;
+            uint32_t found = 0;
             for (uint32_t pos = first; pos < p.pos1; pos += p.splits, ++lt) {
                 const uint32_t acc = lt & 1u;
+                const uint32_t n0 = tile_of(pos) * kNT + half * kCols;
+                // the bias of 32 columns is loaded while the 32 before it are reduced (a tile's
+                // first ones while its product is waited for)
+                const float4* bias = reinterpret_cast<const float4*>(p.bias + n0);
+                float4 bq[2][8];
+                auto fetch_bias = [&](uint32_t cg, float4 (&b)[8]) {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) b[j] = __ldg(bias + cg * 8 + j);
+                };
+                fetch_bias(0, bq[0]);
                 if (!tma_wait(smem_u32(&tfull[acc]), (lt >> 1) & 1u, &failed)) {
                     if (lane == 0) fail();
                     ok = false;
                     break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;");
-                const uint32_t n0 = tile_of(pos) * kNT + half * kCols;
-                const float4* bias = reinterpret_cast<const float4*>(p.bias + n0);
                 const uint32_t taddr = tmem + acc * kNT + half * kCols + ((quarter * 32u) << 16);
                 uint32_t r[2][32];
                 auto fetch = [&](uint32_t cg, uint32_t (&v)[32]) {
@@ -257,11 +271,14 @@ __global__ __launch_bounds__(kThreads, 1) void k_tc_filter(const __grid_constant
 #pragma unroll
                 for (uint32_t cg = 0; cg < kCols / 32; ++cg) {
                     uint32_t(&v)[32] = r[cg & 1];
-                    if (cg + 1 < kCols / 32) fetch(cg + 1, r[(cg + 1) & 1]);
+                    if (cg + 1 < kCols / 32) {
+                        fetch(cg + 1, r[(cg + 1) & 1]);
+                        fetch_bias(cg + 1, bq[(cg + 1) & 1]);
+                    }
                     float gm[4];
 #pragma unroll
                     for (int j = 0; j < 32; j += 4) {
-                        const float4 b = __ldg(bias + cg * 8 + j / 4);
+                        const float4 b = bq[cg & 1][j / 4];
                         const float s0 = __fsub_rn(b.x, __uint_as_float(v[j]));
                         const float s1 = __fsub_rn(b.y, __uint_as_float(v[j + 1]));
                         const float s2 = __fsub_rn(b.z, __uint_as_float(v[j + 2]));
@@ -286,20 +303,18 @@ __global__ __launch_bounds__(kThreads, 1) void k_tc_filter(const __grid_constant
                                      : "memory");
                     }
                     const uint32_t col = n0 + cg * 32;
-                    if (MODE == kTcBelow && fminf(fminf(gm[0], gm[1]), fminf(gm[2], gm[3])) <= thr) {
-#pragma unroll 1
-                        for (int j = 0; j < 32; ++j) {
-                            float s = 0.0f;
+                    if (MODE == kTcBelow) {
+                        // entries are rare: eight columns with one are looked through
 #pragma unroll
-                            for (int t = 0; t < 32; ++t)
-                                if (t == j) s = __uint_as_float(v[t]);
-                            if (s <= thr && col + j < p.N) {
-                                const uint32_t at = atomicAdd(p.count + row, 1u);
-                                if (at < p.cap)
-                                    p.cand[(uint64_t)row * p.cap + at] =
-                                        make_uint2(__float_as_uint(s), p.id0 + col + j);
+                        for (int t = 0; t < 4; ++t)
+                            if (gm[t] <= thr) {
+#pragma unroll
+                                for (int j = 8 * t; j < 8 * t + 8; ++j)
+                                    if (__uint_as_float(v[j]) <= thr && col + j < p.N) {
+                                        if (found < p.seg) list[found] = make_uint2(v[j], p.id0 + col + j);
+                                        ++found;
+                                    }
                             }
-                        }
                     }
                     if (MODE == kTcDense && in) {
                         uint2* out = p.cand + (uint64_t)row * p.cap + (pos - p.pos0) * kNT + half * kCols +
@@ -317,6 +332,7 @@ __global__ __launch_bounds__(kThreads, 1) void k_tc_filter(const __grid_constant
                     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&tempty[acc]))
                                  : "memory");
             }
+            if (MODE == kTcBelow && in) p.count[(uint64_t)row * 2 * p.splits + part] = found;
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
@@ -411,6 +427,12 @@ __global__ __launch_bounds__(kRowWarps * 32) void k_rows_bf16(const float* __res
 
 }  // namespace
 
+// A row tile's columns are split until the items fill the SMs.
+uint32_t tc_filter_splits(uint32_t M) {
+    const uint32_t sms = (uint32_t)sm_count(), mt = (M + 127) / 128;
+    return mt >= sms ? 1u : sms / mt;
+}
+
 bool tc_filter_applies(uint32_t K) { return K > 0 && K <= kMaxResident * 64; }
 
 cudaError_t launch_rows_bf16(const float* X, uint64_t rows, uint32_t d, uint32_t dp, bool seq,
@@ -424,15 +446,15 @@ cudaError_t launch_rows_bf16(const float* X, uint64_t rows, uint32_t d, uint32_t
 }
 
 cudaError_t launch_tc_filter(int mode, const uint16_t* A, uint64_t a_rs, const uint16_t* B,
-                             uint64_t b_rs, TcFilter p, cudaStream_t stream) {
+                             uint64_t b_rs, TcFilter& p, cudaStream_t stream) {
     if (p.M == 0 || p.N == 0 || p.pos1 <= p.pos0) return cudaSuccess;
     CUtensorMap ma, mb;
     if (!encode_bf16_rows(&ma, A, p.M, a_rs, p.K, 128) || !encode_bf16_rows(&mb, B, p.N, b_rs, p.K, kNT))
         return cudaErrorInvalidValue;
     const uint32_t sms = (uint32_t)sm_count(), mt = (p.M + 127) / 128;
-    // a row tile's columns are split until the items fill the SMs
-    p.splits = mt >= sms ? 1u : sms / mt;
+    p.splits = tc_filter_splits(p.M);
     if (p.splits > p.pos1 - p.pos0) p.splits = p.pos1 - p.pos0;
+    p.seg = p.cap / (2 * p.splits);
     const uint32_t items = mt * p.splits, nch = (p.K + 63) / 64;
     const size_t smem = (size_t)a_buffers(nch) * nch * kABytes + kRing * kBBytes + 1024;
     const unsigned grid = items < sms ? items : sms;

@@ -60,3 +60,50 @@ def test_nearest_center_beyond_the_bound():
         oa, od = oracle.nearest_center(c, x)
         assert np.array_equal(a, oa)
         assert np.array_equal(dd.view(np.uint32), od.view(np.uint32))
+
+
+def _knn(base, q, k):
+    import torch
+    ids = torch.empty((len(q), k), dtype=torch.int32, device="cuda")
+    dist = torch.empty((len(q), k), dtype=torch.float32, device="cuda")
+    native.knn(torch.from_numpy(base).cuda(), torch.from_numpy(q).cuda(), k, ids, dist)
+    torch.cuda.synchronize()
+    return ids.cpu().numpy().view(np.uint32), dist.cpu().numpy()
+
+
+def _knn_want(base, q, k):
+    """Small integers: screened scores and distances are exact, so the result is the k
+    smallest (distance, id)."""
+    d2 = ((q * q).sum(1)[:, None] + (base * base).sum(1)[None] - 2.0 * q @ base.T).astype(np.float64)
+    order = np.argsort(d2, axis=1, kind="stable")[:, :k]
+    return order, np.take_along_axis(d2, order, 1)
+
+
+@pytest.mark.parametrize("n,nq,d,k", [(1, 1, 1, 1), (63, 5, 8, 10), (255, 127, 3, 64), (257, 129, 30, 33),
+                                      (2048, 300, 96, 10), (2049, 20, 16, 64), (30000, 260, 20, 64),
+                                      (70001, 40, 96, 10), (3000, 33, 256, 10), (3000, 33, 257, 10)])
+def test_knn_tiles(n, nq, d, k):
+    rng = np.random.default_rng(n + nq)
+    base = rng.integers(0, 4, size=(n, d)).astype(np.float32)
+    q = rng.integers(0, 4, size=(nq, d)).astype(np.float32)
+    ids, dist = _knn(base, q, min(k, n))
+    want, wd = _knn_want(base, q, min(k, n))
+    assert np.array_equal(ids, want)
+    assert np.array_equal(dist, wd)
+
+
+@pytest.mark.parametrize("order", ["sorted", "equal"])
+def test_knn_crowded_lists(order):
+    """Rows in runs of near copies, and all rows equal: more rows below a threshold than a list
+    holds."""
+    rng = np.random.default_rng(1)
+    if order == "equal":
+        base = np.ones((20000, 16), np.float32)
+    else:
+        base = np.repeat(rng.integers(0, 4, size=(6, 16)), 5000, axis=0).astype(np.float32)
+        base[:, 0] += np.arange(30000) % 3
+    q = rng.integers(0, 4, size=(50, 16)).astype(np.float32)
+    ids, dist = _knn(base, q, 64)
+    want, wd = _knn_want(base, q, 64)
+    assert np.array_equal(ids, want)
+    assert np.array_equal(dist, wd)

@@ -46,12 +46,22 @@ struct ProbeNet {
         b3 = W3 + (uint64_t)C * h;
     }
 };
-// Activations and gradients of one training batch (rows <= cap).
+// Buffers of one training batch (rows <= cap), one allocation. The contractions' operands are
+// BF16 with rows padded with zeros to 8 values: each matrix in row order, and transposed (T)
+// where a contraction runs over its rows.
 struct ProbeWork {
     uint32_t cap = 0;
-    float *H1 = nullptr, *Z1 = nullptr, *H2 = nullptr, *Z2 = nullptr, *Z = nullptr, *dZ = nullptr,
-          *dH2 = nullptr, *dH1 = nullptr;
+    uint8_t* block = nullptr;
+    uint16_t *Xb = nullptr, *XT = nullptr, *W1b = nullptr, *W2b = nullptr, *W3b = nullptr,
+             *W2T = nullptr, *W3T = nullptr, *H1b = nullptr, *H1T = nullptr, *H2b = nullptr,
+             *H2T = nullptr, *dZb = nullptr, *dZT = nullptr, *dH2b = nullptr, *dH2T = nullptr,
+             *dH1T = nullptr;
+    // products before bias and GELU, the scores (then their gradient), gradients, row losses
+    float *A1 = nullptr, *A2 = nullptr, *Z = nullptr, *dH1 = nullptr, *dH2 = nullptr,
+          *loss = nullptr;
 };
+// Bytes of the block for n rows; binds the pointers into it when w->block is set.
+size_t probe_work_layout(const ProbeNet& net, uint32_t n, ProbeWork* w);
 
 // Device-resident index. Point arrays are in Puck's "memory order": sorted by
 // (cell id, filter offset, input id), so every coarse cluster is one
@@ -374,8 +384,6 @@ cudaError_t launch_nearest_center_tc(uint32_t dim, const float* cents, uint64_t 
                                      uint64_t n, int32_t* assign, float* dis, cudaStream_t stream);
 
 // Learned probe (probe.cu).
-cudaError_t probe_forward(const ProbeNet& net, const float* X, uint32_t n, float* H1, float* Z1,
-                          float* H2, float* Z2, float* Z, int* err, cudaStream_t st);
 cudaError_t probe_backward(const ProbeNet& net, const float* X, uint32_t n,
                            const uint32_t* labels, uint32_t L, ProbeWork& w, ProbeNet& grad,
                            float* loss_sum, int* err, cudaStream_t st);
@@ -386,6 +394,7 @@ cudaError_t probe_sync_bf16(const ProbeNet& net, cudaStream_t st);
 // X: FP32 queries, or their BF16 copy Xb when not null.
 cudaError_t probe_infer(const ProbeNet& net, const float* X, const uint16_t* Xb, uint32_t n,
                         uint16_t* H1b, uint16_t* H2b, float* Z, int* err, cudaStream_t st);
+// Adam on the FP32 weights; refreshes the BF16 copies.
 cudaError_t probe_adam(ProbeNet& net, const ProbeNet& grad, ProbeNet& m, ProbeNet& v, float lr,
                        uint64_t step, cudaStream_t st);
 cudaError_t launch_probe_select(const ProbeNet& net, const DeviceIndex& ix, uint32_t n,

@@ -13,8 +13,8 @@ struct pgpu_probe {
     float* block = nullptr;  // 4 parameter-sized blocks: weights, gradients, Adam m, Adam v
     uint16_t* bf16 = nullptr;  // BF16 copies of W1, W2, W3
     pgpu::ProbeWork work;
-    float* loss = nullptr;   // device scalar
-    int* err = nullptr;      // device flag of the tensor-core waits
+    float* loss = nullptr;   // device scalar, followed by
+    int* err = nullptr;      // the flag of the tensor-core waits
     uint64_t step = 0;
     cudaStream_t stream = nullptr;
     std::mutex mu;
@@ -33,27 +33,21 @@ int cuda_fail(cudaError_t e, const char* what) {
 }
 
 void free_work(pgpu::ProbeWork* w) {
-    float* ptrs[] = {w->H1, w->Z1, w->H2, w->Z2, w->Z, w->dZ, w->dH2, w->dH1};
-    for (float* p : ptrs)
-        if (p) cudaFree(p);
+    if (w->block) cudaFree(w->block);
     *w = pgpu::ProbeWork();
 }
 
 cudaError_t ensure_work(pgpu_probe* p, uint32_t n) {
     if (p->work.cap >= n) return cudaSuccess;
     free_work(&p->work);
-    const uint64_t h = p->net.h, C = p->net.C;
     pgpu::ProbeWork& w = p->work;
-    cudaError_t e = cudaSuccess;
-    float** hs[] = {&w.H1, &w.Z1, &w.H2, &w.Z2, &w.dH2, &w.dH1};
-    for (float** q : hs)
-        if (e == cudaSuccess) e = cudaMalloc((void**)q, sizeof(float) * n * h);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&w.Z, sizeof(float) * n * C);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&w.dZ, sizeof(float) * n * C);
+    const size_t bytes = pgpu::probe_work_layout(p->net, n, &w);
+    cudaError_t e = cudaMalloc((void**)&w.block, bytes);
     if (e != cudaSuccess) {
         free_work(&w);
         return e;
     }
+    pgpu::probe_work_layout(p->net, n, &w);
     w.cap = n;
     return cudaSuccess;
 }
@@ -62,23 +56,22 @@ cudaError_t ensure_work(pgpu_probe* p, uint32_t n) {
 int run_backward(pgpu_probe* p, const float* x, const uint32_t* labels, uint32_t n, uint32_t L) {
     cudaError_t e = ensure_work(p, n);
     if (e != cudaSuccess) return cuda_fail(e, "probe work buffers");
-    cudaMemsetAsync(p->loss, 0, sizeof(float), p->stream);
-    cudaMemsetAsync(p->err, 0, sizeof(int), p->stream);
+    cudaMemsetAsync(p->loss, 0, sizeof(float) + sizeof(int), p->stream);
     e = pgpu::probe_backward(p->net, x, n, labels, L, p->work, p->grad, p->loss, p->err, p->stream);
     if (e != cudaSuccess) return cuda_fail(e, "probe backward");
     return PGPU_OK;
 }
 
 int finish(pgpu_probe* p, float* loss) {
-    float l = 0.0f;
-    int flag = 0;
-    cudaError_t e = cudaMemcpyAsync(&l, p->loss, sizeof(float), cudaMemcpyDeviceToHost, p->stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(&flag, p->err, sizeof(int), cudaMemcpyDeviceToHost, p->stream);
+    struct {
+        float loss;
+        int err;
+    } got = {0.0f, 0};
+    cudaError_t e = cudaMemcpyAsync(&got, p->loss, sizeof(got), cudaMemcpyDeviceToHost, p->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(p->stream);
     if (e != cudaSuccess) return cuda_fail(e, "probe step");
-    if (flag) return pgpu::set_last_error(PGPU_E_TIMEOUT, "tensor-core wait expired");
-    if (loss) *loss = l;
+    if (got.err) return pgpu::set_last_error(PGPU_E_TIMEOUT, "tensor-core wait expired");
+    if (loss) *loss = got.loss;
     return PGPU_OK;
 }
 
@@ -110,10 +103,10 @@ int pgpu_probe_create(uint32_t dim, uint32_t hidden, uint32_t clusters, uint64_t
     cudaError_t e = cudaMalloc((void**)&p->block, sizeof(float) * np * 4);
     const uint64_t nw = (uint64_t)hidden * dim + (uint64_t)hidden * hidden + (uint64_t)clusters * hidden;
     if (e == cudaSuccess) e = cudaMalloc((void**)&p->bf16, sizeof(uint16_t) * nw);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&p->loss, sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&p->err, sizeof(int));
+    if (e == cudaSuccess) e = cudaMalloc((void**)&p->loss, sizeof(float) + sizeof(int));
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) {
+        p->err = reinterpret_cast<int*>(p->loss + 1);
         p->net.bind(p->block);
         p->grad.bind(p->block + np);
         p->m.bind(p->block + 2 * np);
@@ -131,7 +124,6 @@ int pgpu_probe_create(uint32_t dim, uint32_t hidden, uint32_t clusters, uint64_t
         if (p->block) cudaFree(p->block);
         if (p->bf16) cudaFree(p->bf16);
         if (p->loss) cudaFree(p->loss);
-        if (p->err) cudaFree(p->err);
         if (p->stream) cudaStreamDestroy(p->stream);
         delete p;
         return rc;
@@ -148,7 +140,6 @@ int pgpu_probe_destroy(pgpu_probe* p) {
     cudaFree(p->block);
     cudaFree(p->bf16);
     cudaFree(p->loss);
-    cudaFree(p->err);
     cudaStreamDestroy(p->stream);
     delete p;
     return PGPU_OK;
@@ -173,7 +164,6 @@ int pgpu_probe_train_step(pgpu_probe* p, const float* queries, const uint32_t* l
     if (int rc = run_backward(p, queries, labels, n, L)) return rc;
     p->step += 1;
     cudaError_t e = pgpu::probe_adam(p->net, p->grad, p->m, p->v, lr, p->step, p->stream);
-    if (e == cudaSuccess) e = pgpu::probe_sync_bf16(p->net, p->stream);
     if (e != cudaSuccess) return cuda_fail(e, "probe update");
     return finish(p, loss);
 }
@@ -202,8 +192,7 @@ int pgpu_probe_forward(pgpu_probe* p, const float* queries, uint32_t n, float* s
     if (e != cudaSuccess) return cuda_fail(e, "probe work buffers");
     cudaMemsetAsync(p->err, 0, sizeof(int), p->stream);
     // the search's own inference path: BF16 weights and activations
-    e = pgpu::probe_infer(p->net, queries, nullptr, n, reinterpret_cast<uint16_t*>(p->work.H1),
-                          reinterpret_cast<uint16_t*>(p->work.H2), scores, p->err, p->stream);
+    e = pgpu::probe_infer(p->net, queries, nullptr, n, p->work.H1b, p->work.H2b, scores, p->err, p->stream);
     if (e != cudaSuccess) return cuda_fail(e, "probe forward");
     return finish(p, nullptr);
 }

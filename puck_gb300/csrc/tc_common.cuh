@@ -38,6 +38,15 @@ __device__ __forceinline__ bool tma_wait(uint32_t bar, uint32_t parity, const vo
     return false;
 }
 
+__device__ __forceinline__ float gelu_f(float x) {
+    return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f));
+}
+__device__ __forceinline__ float gelu_grad_f(float x) {
+    const float cdf = 0.5f * (1.0f + erff(x * 0.70710678118654752f));
+    const float pdf = 0.39894228040143268f * expf(-0.5f * x * x);
+    return cdf + x * pdf;
+}
+
 // 2-D BF16 tensor map of rows x K values at p, rows rs elements apart (16-byte aligned), box
 // 64 (K) x box_rows, 128-byte swizzle, zero fill past the ends.
 bool encode_bf16_rows(CUtensorMap* map, const uint16_t* p, uint64_t rows, uint64_t rs, uint32_t K,

@@ -170,15 +170,6 @@ __device__ __forceinline__ void stage_operand_async(uint8_t* tile, const TcOpera
     }
 }
 
-__device__ __forceinline__ float gelu_f(float x) {
-    return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f));
-}
-__device__ __forceinline__ float gelu_grad_f(float x) {
-    const float cdf = 0.5f * (1.0f + erff(x * 0.70710678118654752f));
-    const float pdf = 0.39894228040143268f * expf(-0.5f * x * x);
-    return cdf + x * pdf;
-}
-
 template <int EPI>
 __device__ __forceinline__ float epilogue(float acc, uint32_t i, uint32_t j, const TcEpilogue& ep) {
     if (EPI == TC_EPI_SCORE) return __fsub_rn(ep.bias[j], acc);

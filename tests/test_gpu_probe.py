@@ -58,6 +58,41 @@ def test_probe_gradients_match_oracle():
     p.close()
 
 
+# Rows and columns at and around the tiles of the copies (64) and of the contractions (128 and
+# chunks of 64), rows that are not 16-byte aligned, split products, a batch of one, repeated and
+# missing labels. Bounds as above: the operands are rounded to BF16 at the same places.
+@pytest.mark.parametrize("d,h,C,n,L", [(30, 50, 129, 1, 1), (30, 50, 129, 65, 3), (64, 64, 64, 64, 1),
+                                       (96, 129, 7, 127, 40), (8, 256, 1000, 129, 10),
+                                       (96, 512, 300, 1500, 10), (33, 127, 4100, 257, 2)])
+def test_probe_gradients_tile_edges(d, h, C, n, L):
+    import torch
+    p = native.Probe(d, h, C, seed=5)
+    rng = np.random.default_rng(d + h + C + n)
+    X = rng.normal(size=(n, d)).astype(np.float32)
+    labels = rng.integers(0, C, size=(n, L)).astype(np.uint32)
+    labels[n // 2:, L // 2:] = labels[n // 2:, :1]
+    labels[3::5] = probe_mlp.NO_LABEL
+    xt = torch.from_numpy(X).cuda()
+    lt = torch.from_numpy(labels.view(np.int32)).cuda()
+    torch.cuda.synchronize()
+    scores = torch.empty(n, C, device="cuda")
+    for step in range(2):
+        p.train_step(xt, lt, 1e-2)
+        params = p.get_params()
+        loss, g = p.gradients(xt, lt)
+        oloss, og = probe_mlp.forward_backward(params, X, labels, d, h, C, bf16=True)
+        assert abs(loss - oloss) <= 1e-3 * max(1.0, abs(oloss))
+        for gg, oo in zip(p.split(g), p.split(og)):
+            gg = gg.astype(np.float64)
+            assert np.all(np.abs(gg - oo) <= 2e-2 * np.abs(oo).max() + 1e-7)
+            assert np.linalg.norm(gg - oo) <= 1e-2 * np.linalg.norm(oo) + 1e-9
+        # the buffers are shared with inference, whose rows are not padded; a smaller batch follows
+        p.forward(xt, scores)
+        xt, lt, X, labels = xt[:n - n // 3], lt[:n - n // 3], X[:n - n // 3], labels[:n - n // 3]
+        scores = scores[:n - n // 3]
+    p.close()
+
+
 def test_knn_matches_fp64_scan():
     import torch
     rng = np.random.default_rng(1)

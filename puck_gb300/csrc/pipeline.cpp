@@ -35,34 +35,20 @@ void ensure_max_dynamic_smem(const void* kernel, int bytes) {
 void free_scratch(Scratch* s) {
     void* ptrs[] = {s->q, s->qb, s->qnorm, s->status, s->dots, s->cdist, s->ctag, s->fdist,
                     s->ftag, s->hdist, s->htag, s->hcnt, s->counters, s->tc_err,
-                    s->ph1, s->ph2, s->pconf, s->pz, s->order, s->wbucket, s->ulist, s->ucount,
-                    s->tbuf, s->qcnt, s->qoff, s->qflag, s->cut};
+                    s->ph1, s->ph2, s->pconf, s->pz, s->order, s->wbin, s->ulist, s->ucount,
+                    s->todo, s->ntodo};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     *s = Scratch();
-}
-
-// Split scan buffer: room for 40960 record distances per query of the batch (about
-// 1.6 times the mean record count of a coarse cluster at 100M points and 4000
-// clusters), at least 2^20 and at most 2^30. A query whose records do not fit runs
-// the fused scan kernel instead.
-uint64_t split_capacity(const DeviceIndex& ix, const SearchConfig& cfg, uint32_t B) {
-    if (cfg.mode != PGPU_MODE_SCAN || !scan_split_possible(ix, cfg.filter_keep())) return 0;
-    uint64_t c = (uint64_t)B * 40960ull;
-    if (c < (1ull << 20)) c = 1ull << 20;
-    if (c > (1ull << 30)) c = 1ull << 30;
-    return c;
 }
 
 uint64_t scratch_bytes(const DeviceIndex& ix, const SearchConfig& cfg, uint32_t B) {
     const uint64_t P = cfg.coarse_slots(ix.C), T = cfg.filter_keep();
     const uint64_t probe = cfg.probe ? (uint64_t)B * (cfg.probe->h * 4 + 8 + ix.C * 4ull) + 4 : 0;
     const uint64_t fine_order = cfg.mode == PGPU_MODE_EXACT ? (uint64_t)B * ix.F * 8 : 8;
-    const uint64_t tables = cfg.mode == PGPU_MODE_SCAN ? (uint64_t)B * 5 : 0;  // launch order
-    const uint64_t tcap = split_capacity(ix, cfg, B);
-    const uint64_t split = tcap ? tcap * 4 + (uint64_t)B * (12 + sizeof(SplitCut)) : 0;
+    const uint64_t tables = cfg.mode == PGPU_MODE_SCAN ? (uint64_t)B * 10 + 4 : 0;  // launch order
     return (uint64_t)B * (ix.d * 6 + 4 + 4 + std::max(ix.C, ix.F) * 4ull + P * 8 + T * 8 + 4) +
-           fine_order + tables + split + probe + kNumWalkCounters * 8 + 4;
+           fine_order + tables + probe + kNumWalkCounters * 8 + 4;
 }
 
 int alloc_scratch(const DeviceIndex& ix, const SearchConfig& cfg, uint32_t B, Scratch* out,
@@ -94,16 +80,9 @@ int alloc_scratch(const DeviceIndex& ix, const SearchConfig& cfg, uint32_t B, Sc
     PGPU_ALLOC(s.tc_err, 1);
     if (cfg.mode == PGPU_MODE_SCAN) {
         PGPU_ALLOC(s.order, B);
-        PGPU_ALLOC(s.wbucket, B);
-        const uint64_t tcap = split_capacity(ix, cfg, B);
-        if (tcap) {
-            PGPU_ALLOC(s.tbuf, tcap);
-            PGPU_ALLOC(s.qcnt, B);
-            PGPU_ALLOC(s.qoff, B);
-            PGPU_ALLOC(s.qflag, B);
-            PGPU_ALLOC(s.cut, B);
-            s.tcap = tcap;
-        }
+        PGPU_ALLOC(s.wbin, B);
+        PGPU_ALLOC(s.todo, B);
+        PGPU_ALLOC(s.ntodo, 1);
     }
     if (cfg.probe) {
         PGPU_ALLOC(s.ulist, B);
@@ -185,7 +164,6 @@ cudaError_t run_pipeline(const DeviceIndex& ix, const SearchConfig& cfg, Scratch
         k = 7;
     } else {
         PGPU_STEP(launch_scan_order(ix, n, s, st), "scan order");
-        PGPU_STEP(launch_scan_prepare(ix, n, s, bf16, st), "scan prepare");
     }
     mark(5);
     if (cfg.mode == PGPU_MODE_EXACT) {
@@ -203,11 +181,11 @@ cudaError_t run_pipeline(const DeviceIndex& ix, const SearchConfig& cfg, Scratch
     }
     mark(8);
 #undef PGPU_STEP
-    // scan mode adds the two launch-order kernels, and the split scan three more
-    // (k_split_counts, k_split_offsets, k_scan_score; the fused kernel is counted in k)
+    // scan mode adds the two launch-order kernels, and the split scan one more
+    // (k_scan_score; the fused kernel is counted in k)
     if (launched)
         *launched = k + probe_kernels +
-                    (cfg.mode == PGPU_MODE_SCAN ? 2 + (scan_split_applies(ix, s) ? 3 : 0) : 0);
+                    (cfg.mode == PGPU_MODE_SCAN ? 2 + (scan_split_applies(ix, s) ? 1 : 0) : 0);
     return cudaSuccess;
 }
 

@@ -52,6 +52,7 @@ struct RerankParams {
     const float* q;
     const float* qnorm;
     const int32_t* status;
+    const uint32_t* order;  // query of each block (scan mode: queries of one cluster together), or null
     const float* hdist;
     int sort_ties;  // scan mode: replay ties in the filter's (t, memory id) order
     const uint32_t* htag;
@@ -242,7 +243,7 @@ __global__ __launch_bounds__(kThreads) void k_rerank(RerankParams p) {
     __shared__ uint32_t sel_hist[256];
     __shared__ uint32_t sel_state[2];
     __shared__ uint32_t sel_count;
-    const uint32_t qi = blockIdx.x, topk = p.topk;
+    const uint32_t qi = p.order ? p.order[blockIdx.x] : blockIdx.x, topk = p.topk;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     float* od = p.out_dist + (uint64_t)qi * topk;
     uint32_t* oi = p.out_ids + (uint64_t)qi * topk;
@@ -429,6 +430,7 @@ __device__ __forceinline__ float screen_bound(float dt, float xabs, uint32_t d) 
 struct ScreenParams {
     const float* q;
     const int32_t* status;
+    const uint32_t* order;
     const float* hdist;
     const uint32_t* htag;
     const uint32_t* hcnt;
@@ -455,7 +457,7 @@ __global__ __launch_bounds__(kScreenThreads, PGPU_RERANK_SCREEN_MIN_BLOCKS) void
     __shared__ uint32_t hist[256];
     __shared__ uint32_t state[2];
     __shared__ uint32_t wcount;
-    const uint32_t qi = blockIdx.x, topk = p.topk, d = p.d;
+    const uint32_t qi = p.order ? p.order[blockIdx.x] : blockIdx.x, topk = p.topk, d = p.d;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     float* od = p.out_dist + (uint64_t)qi * topk;
     uint32_t* oi = p.out_ids + (uint64_t)qi * topk;
@@ -679,6 +681,7 @@ cudaError_t launch_rerank(const DeviceIndex& ix, const SearchConfig& cfg, uint32
     p.q = s.q;
     p.qnorm = s.qnorm;
     p.status = s.status;
+    p.order = s.order;
     p.hdist = s.hdist;
     p.sort_ties = cfg.mode == PGPU_MODE_SCAN ? 1 : 0;
     p.pq_codebook = ix.pq_codebook;
@@ -723,6 +726,7 @@ cudaError_t launch_rerank_screen(const DeviceIndex& ix, uint32_t n, uint32_t top
     ScreenParams p;
     p.q = s.q;
     p.status = s.status;
+    p.order = s.order;
     p.hdist = s.hdist;
     p.htag = s.htag;
     p.hcnt = s.hcnt;

@@ -59,6 +59,8 @@
 // fetched while the previous round is scored.
 #include <cuda_fp16.h>
 
+#include <type_traits>
+
 #include "device_common.cuh"
 #include "pgpu_internal.h"
 
@@ -116,7 +118,9 @@ struct ScanParams {
     int* err;                   // set when a bulk copy's wait expired
     const uint32_t* ins_cl_start;  // realtime: [C+1] inserted records per cluster, or null
     const uint32_t* ins_cl_ids;    // their memory ids
-    const uint32_t* done;          // [B] 1: the split scan has answered the query, or null
+    const uint32_t* todo;          // k_scan_il: the queries the split scan left, or null (all, in order)
+    const uint32_t* ntodo;         // their number (device)
+    uint32_t n;
     uint32_t d, C, F, nsq, lsq, code_stride, P, T, cap;
     float codebook_max;
 };
@@ -723,7 +727,6 @@ __global__ __launch_bounds__(kThreads, PGPU_SCAN_MIN_BLOCKS) void k_scan_select(
     float* srow = HALF ? reinterpret_cast<float*>(luth + nsq * 256) : lut + nsq * 256;
     float* qv = srow + F;                  // [d]
 
-    if (p.done && p.done[qi]) return;  // answered by the split scan
     if (p.status[qi] != 0) {
         if (tid == 0) p.hcnt[qi] = 0;
         return;
@@ -888,63 +891,82 @@ __device__ __forceinline__ bool il_wait(uint32_t bar, uint32_t parity) {
 // codeword's subspaces go in two halves, a thread per half (NT = 512) or both halves
 // by one thread (NT = 256). All NT threads; one barrier inside (after the staging),
 // none after the expansion.
+// il_load_half issues the codebook loads of a thread's first half (lsq 4), which need
+// no query: the caller does so before it reads anything else.
+template <int NSQ>
+__device__ __forceinline__ void il_load_half(const float* __restrict__ codebook, uint32_t h2,
+                                             float4 (&y)[NSQ / 2]) {
+    const float4* cb4 =
+        reinterpret_cast<const float4*>(codebook) + h2 * (NSQ / 2) * 256u + (threadIdx.x & 255u);
+#pragma unroll
+    for (int m = 0; m < NSQ / 2; ++m) y[m] = __ldg(cb4 + m * 256);
+}
+template <int NSQ>
+__device__ __forceinline__ void il_stage_half(float* stage, const float* qv, uint32_t h2,
+                                              const float4 (&y)[NSQ / 2]) {
+    const float4* q4 = reinterpret_cast<const float4*>(qv) + h2 * (NSQ / 2);
+    float* out = stage + h2 * (NSQ / 2) * 257u + (threadIdx.x & 255u);
+#pragma unroll
+    for (int m = 0; m < NSQ / 2; ++m) {
+        const float4 x = q4[m];
+        const float t0 = __fsub_rn(x.x, y[m].x), t1 = __fsub_rn(x.y, y[m].y);
+        const float t2 = __fsub_rn(x.z, y[m].z), t3 = __fsub_rn(x.w, y[m].w);
+        out[m * 257] = __fadd_rn(__fadd_rn(__fmul_rn(t0, t0), __fmul_rn(t1, t1)),
+                                 __fadd_rn(__fmul_rn(t2, t2), __fmul_rn(t3, t3)));
+    }
+}
+
 template <int NSQ, bool HALF, int NT, bool WIDE = false>
 __device__ __forceinline__ void il_build_table(unsigned char* tab, float* stage, const float* qv,
                                                const float* __restrict__ codebook, uint32_t lsq,
-                                               int lut_e) {
+                                               int lut_e, float4 (&y)[NSQ / 2]) {
     static_assert(NT % 256 == 0, "a thread per codeword and half");
     const int tid = threadIdx.x;
-    for (uint32_t h2 = tid >> 8; h2 < 2; h2 += NT / 256) {
-        const uint32_t j = tid & 255u;
-        const int mh = (int)h2 * (NSQ / 2);
-        if (lsq == 4) {
-            const float4* cb4 = reinterpret_cast<const float4*>(codebook);
-#pragma unroll
-            for (int m0 = 0; m0 < NSQ / 2; m0 += 2) {
-                float4 y[2];
-#pragma unroll
-                for (int u = 0; u < 2; ++u) y[u] = __ldg(cb4 + (uint64_t)(mh + m0 + u) * 256 + j);
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    const int m = mh + m0 + u;
-                    const float* x = qv + m * 4;
-                    const float t0 = __fsub_rn(x[0], y[u].x), t1 = __fsub_rn(x[1], y[u].y);
-                    const float t2 = __fsub_rn(x[2], y[u].z), t3 = __fsub_rn(x[3], y[u].w);
-                    stage[m * 257 + j] = __fadd_rn(__fadd_rn(__fmul_rn(t0, t0), __fmul_rn(t1, t1)),
-                                                   __fadd_rn(__fmul_rn(t2, t2), __fmul_rn(t3, t3)));
-                }
-            }
+    if (lsq == 4) {
+        if (NT == 256) {
+            float4 z[NSQ / 2];
+            il_load_half<NSQ>(codebook, 1, z);
+            il_stage_half<NSQ>(stage, qv, 0, y);
+            il_stage_half<NSQ>(stage, qv, 1, z);
         } else {
+            il_stage_half<NSQ>(stage, qv, tid >> 8, y);
+        }
+    } else {
+        for (uint32_t h2 = tid >> 8; h2 < 2; h2 += NT / 256) {
+            const uint32_t j = tid & 255u;
+            const int mh = (int)h2 * (NSQ / 2);
             for (int m = mh; m < mh + NSQ / 2; ++m)
                 stage[m * 257 + j] =
                     l2sqr_sse(qv + m * lsq, codebook + ((uint64_t)m * 256 + j) * lsq, lsq);
         }
     }
     __syncthreads();
-    if (HALF && WIDE) {
-        // each FP16 entry in its own 4-byte slot (the FP32 table's addresses)
-        const float scale = ldexpf(1.0f, lut_e);
-        uint32_t* tw = reinterpret_cast<uint32_t*>(tab);
-        for (uint32_t w = tid; w < 256 * 64; w += NT) {
-            const uint32_t c = w >> 6, m = w & 63;
-            const float v = m < NSQ + 31 ? stage[(m % NSQ) * 257 + c] : 0.0f;
-            tw[w] = (uint32_t)__half_as_ushort(__float2half_rn(v * scale));
-        }
-    } else if (HALF) {
-        const float scale = ldexpf(1.0f, lut_e);
-        uint32_t* tw = reinterpret_cast<uint32_t*>(tab);
-        for (uint32_t w = tid; w < 256 * 32; w += NT) {
-            const uint32_t c = w >> 5, m0 = (w & 31) * 2;
-            const float v0 = m0 < NSQ + 31 ? stage[(m0 % NSQ) * 257 + c] : 0.0f;
-            const float v1 = m0 + 1 < NSQ + 31 ? stage[((m0 + 1) % NSQ) * 257 + c] : 0.0f;
-            const __half2 h = __halves2half2(__float2half_rn(v0 * scale), __float2half_rn(v1 * scale));
-            tw[w] = *reinterpret_cast<const uint32_t*>(&h);
+    // a thread keeps its columns and walks down the rows: one load and one store per entry
+    // (columns past NSQ + 30 are never read)
+    const float scale = HALF ? ldexpf(1.0f, lut_e) : 1.0f;
+    if (HALF && !WIDE) {
+        const uint32_t m0 = (tid & 31) * 2;
+        if (m0 < NSQ + 31) {
+            const float* s0 = stage + (m0 % NSQ) * 257;
+            const float* s1 = stage + ((m0 + 1) % NSQ) * 257;
+            uint32_t* tw = reinterpret_cast<uint32_t*>(tab) + (tid & 31);
+#pragma unroll 8
+            for (uint32_t c = tid >> 5; c < 256; c += NT / 32) {
+                const __half2 h = __halves2half2(__float2half_rn(s0[c] * scale),
+                                                 __float2half_rn(s1[c] * scale));
+                tw[c * 32] = *reinterpret_cast<const uint32_t*>(&h);
+            }
         }
     } else {
-        float* tf = reinterpret_cast<float*>(tab);
-        for (uint32_t w = tid; w < 256 * 64; w += NT) {
-            const uint32_t c = w >> 6, m = w & 63;
-            tf[w] = m < NSQ + 31 ? stage[(m % NSQ) * 257 + c] : 0.0f;
+        const uint32_t m = tid & 63;
+        if (m < NSQ + 31) {
+            const float* src = stage + (m % NSQ) * 257;
+            uint32_t* tw = reinterpret_cast<uint32_t*>(tab) + m;
+#pragma unroll 8
+            for (uint32_t c = tid >> 6; c < 256; c += NT / 64)
+                // WIDE: each FP16 entry in its own 4-byte slot (the FP32 table's addresses)
+                tw[c * 64] = HALF ? (uint32_t)__half_as_ushort(__float2half_rn(src[c] * scale))
+                                  : __float_as_uint(src[c]);
         }
     }
 }
@@ -980,8 +1002,9 @@ __device__ __forceinline__ void il_score(const unsigned char* tab, const float* 
                          : *reinterpret_cast<const unsigned short*>(tab + (addr >> 1) + 2 * s2);
                 asm("add.f32.f16 %0, %1, %0;" : "+f"(a[j][s2 & 3]) : "h"(h));
             } else {
-                a[j][s2 & 3] =
-                    __fadd_rn(a[j][s2 & 3], *reinterpret_cast<const float*>(tab + addr + 4 * s2));
+                // the first four entries start the sums: an entry is never -0, so 0 + x is x
+                const float x = *reinterpret_cast<const float*>(tab + addr + 4 * s2);
+                a[j][s2 & 3] = s2 < 4 ? x : __fadd_rn(a[j][s2 & 3], x);
             }
         }
     }
@@ -1009,7 +1032,6 @@ __global__ __launch_bounds__(IlShape<HALF>::kThreads, IlShape<HALF>::kMinBlocks)
     __shared__ ScanState st;
     __shared__ __align__(8) uint64_t full[kIlStages];
     __shared__ int il_failed;
-    const uint32_t qi = p.order[blockIdx.x];
     const int tid = threadIdx.x;
     const uint32_t F = p.F, T = p.T, cap = p.cap;
     unsigned char* tab = smem;  // the rotated table, at offset 0
@@ -1021,13 +1043,7 @@ __global__ __launch_bounds__(IlShape<HALF>::kThreads, IlShape<HALF>::kMinBlocks)
     uint64_t* keys = reinterpret_cast<uint64_t*>(rest + il_srow_bytes(F));  // [cap]
     uint32_t* hist = reinterpret_cast<uint32_t*>(keys + cap);              // [kHistBins]
 
-    if (p.done && p.done[qi]) return;  // answered by the split scan
-    if (p.status[qi] != 0) {
-        if (tid == 0) p.hcnt[qi] = 0;
-        return;
-    }
-    const long long t_start = clock64();
-    // rounds issued and consumed over the whole block (slot g % S, parity (g / S) & 1)
+    // rounds issued and consumed over all the block's queries (slot g % S, parity (g / S) & 1)
     uint32_t g_issued = 0, g_done = 0;
     auto bar_of = [&](uint32_t g) { return (uint32_t)__cvta_generic_to_shared(&full[g % kIlStages]); };
     // thread 0: bulk copy of record blocks [blk0, blk0 + nblk) into round g's slot
@@ -1048,210 +1064,227 @@ __global__ __launch_bounds__(IlShape<HALF>::kThreads, IlShape<HALF>::kMinBlocks)
         for (int i = 0; i < kIlStages; ++i)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar_of(i)), "r"(1u));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        st.tau = kKeyMax;
-        st.count = 0;
-        st.evaluated = st.looked = st.passed = 0;
-        st.cyc_rounds = st.cyc_compact = st.n_compact = st.n_records = 0;
         il_failed = 0;
     }
-    // the first cluster's first rounds go out before the table is built
-    uint32_t primed_blk0 = 0, primed_blocks = 0;
-    if (tid == 0) {
-        const uint32_t c = p.ctag[(uint64_t)qi * p.P];
-        if (c < p.C) {
-            const uint32_t r0 = p.cell_start[(uint64_t)c * F], r1 = p.cell_start[(uint64_t)c * F + F];
-            if (r1 > r0) {
-                const uint32_t b0 = r0 >> 5, nblk = ((r1 - 1) >> 5) - b0 + 1;
-                primed_blk0 = b0;
-                for (uint32_t k = 0; k < (uint32_t)kIlStages && k * kIlBlocksPerRound < nblk; ++k) {
-                    const uint32_t m = min(kIlBlocksPerRound, nblk - k * kIlBlocksPerRound);
-                    issue(g_issued++, (uint64_t)b0 + k * kIlBlocksPerRound, m);
-                    primed_blocks += m;
-                }
-            }
+    const uint32_t nq = p.todo ? *p.ntodo : p.n;
+    for (uint32_t qb = blockIdx.x; qb < nq; qb += gridDim.x) {
+        const uint32_t qi = p.todo ? p.todo[qb] : p.order[qb];
+        if (p.status[qi] != 0) {
+            if (tid == 0) p.hcnt[qi] = 0;
+            continue;
         }
-    }
-    for (uint32_t i = tid; i < p.d; i += kIlThreads) qv[i] = p.q[(uint64_t)qi * p.d + i];
-    const float* fdk = p.fd_by_fine + (uint64_t)qi * F;
-    // the first cluster's stationary row and this query's fine terms are loaded now,
-    // so their latency overlaps the table build (srow is written after it)
-    constexpr int kPre = 2;  // float4 per thread and row (F <= kPre * 4 * kIlThreads)
-    const uint32_t c_first = p.ctag[(uint64_t)qi * p.P];
-    const bool pre = c_first < p.C && (F & 3u) == 0 && F <= kPre * 4 * kIlThreads;
-    float4 pre_st[kPre], pre_fd[kPre];
-#pragma unroll
-    for (int u = 0; u < kPre; ++u) {
-        const uint32_t i = tid + u * kIlThreads;
-        if (pre && i < (F >> 2)) {
-            pre_st[u] = __ldg(reinterpret_cast<const float4*>(p.stationary + (uint64_t)c_first * F) + i);
-            pre_fd[u] = __ldg(reinterpret_cast<const float4*>(fdk) + i);
-        }
-    }
-    const int lut_e = HALF ? half_lut_exponent(p.qnorm[qi], p.codebook_max) : 0;
-    const float inv_scale = HALF ? ldexpf(1.0f, -lut_e) : 1.0f;
-    __syncthreads();
-    il_build_table<NSQ, HALF, kIlThreads>(tab, stage, qv, p.codebook, p.lsq, lut_e);
-    unsigned long long my_eval = 0, my_pass = 0;
-    const long long t_pro = clock64();
-
-    auto score_records = [&](const uint2 (&gr)[kIlRec][NG], const float (&off)[kIlRec],
-                             const uint32_t (&fine)[kIlRec], const uint32_t (&mr)[kIlRec],
-                             float (&t)[kIlRec]) {
-        il_score<NSQ, HALF, kIlRec>(tab, srow, gr, off, fine, mr, inv_scale, t);
-    };
-
-    for (uint32_t l = 0; l < p.P && !il_failed; ++l) {
-        if (!scan_cluster_begin(p, st, qi, l)) break;  // (its first barrier ends the table)
-        const uint32_t r0 = st.r0, r1 = st.r1, i0 = st.i0, ni = st.i1 - st.i0;
-        if (r1 - r0 + ni == 0) continue;
-        if (tid == 0) st.n_records += r1 - r0 + ni;
-        if (l == 0 && pre) {
-            // srow from the rows loaded before the table build
-            const float cdl = st.cdl;
-            float4* s4 = reinterpret_cast<float4*>(srow);
-#pragma unroll
-            for (int u = 0; u < kPre; ++u) {
-                const uint32_t i = tid + u * kIlThreads;
-                if (i < (F >> 2)) {
-                    const float4 a = pre_st[u], b = pre_fd[u];
-                    s4[i] = make_float4(2.0f * __fadd_rn(__fadd_rn(cdl, a.x), b.x),
-                                        2.0f * __fadd_rn(__fadd_rn(cdl, a.y), b.y),
-                                        2.0f * __fadd_rn(__fadd_rn(cdl, a.z), b.z),
-                                        2.0f * __fadd_rn(__fadd_rn(cdl, a.w), b.w));
-                }
-            }
-            __syncthreads();
-        } else {
-            scan_fill_srow(p, srow, fdk, st.c, st.cdl);
-        }
-        uint32_t b0 = 0, nblk = 0, rounds = 0;
-        if (r1 > r0) {
-            b0 = r0 >> 5;
-            nblk = ((r1 - 1) >> 5) - b0 + 1;
-            rounds = (nblk + kIlBlocksPerRound - 1) / kIlBlocksPerRound;
-        }
-        // rounds of this cluster already in flight (the first cluster's, primed)
-        uint32_t sent = (l == 0 && primed_blocks > 0 && primed_blk0 == b0)
-                            ? (primed_blocks + kIlBlocksPerRound - 1) / kIlBlocksPerRound
-                            : 0;
+        const long long t_start = clock64();
+        __syncthreads();  // the previous query's buffers are no longer read
         if (tid == 0) {
-            for (; sent < rounds && sent < (uint32_t)kIlStages; ++sent)
-                issue(g_issued++, (uint64_t)b0 + sent * kIlBlocksPerRound,
-                      min(kIlBlocksPerRound, nblk - sent * kIlBlocksPerRound));
+            st.tau = kKeyMax;
+            st.count = 0;
+            st.evaluated = st.looked = st.passed = 0;
+            st.cyc_rounds = st.cyc_compact = st.n_compact = st.n_records = 0;
         }
-        sent = rounds < (uint32_t)kIlStages ? rounds : (uint32_t)kIlStages;
-        g_issued = g_done + sent;  // every thread tracks the count thread 0 issued
-        const uint32_t blk = tid >> 5, lane = tid & 31;
-        for (uint32_t k = 0; k < rounds; ++k) {
-            const long long t_round = clock64();
-            const uint64_t tau = st.tau;
-            // tau as (float, id): key(t, id) < tau iff t < tau_f, or t == tau_f and
-            // id < tau_id (float compares treat -0 as +0, as the keys do; a bound
-            // whose float part is the key of -0 keeps exactly the t < 0)
-            float tau_f = tau == kKeyMax ? __int_as_float(0x7f800000) : key_value(tau);
-            uint32_t tau_id = tau == kKeyMax ? 0xFFFFFFFFu : (uint32_t)tau;
-            if ((uint32_t)(tau >> 32) == 0x7FFFFFFFu) {
-                tau_f = 0.0f;
-                tau_id = 0;
-            }
-            const uint32_t g = g_done;
-            if (!il_wait(bar_of(g), (g / kIlStages) & 1u)) {
-                if (lane == 0) atomicExch(&il_failed, 1);
-            }
-            uint2 gr[kIlRec][NG];
-            float off[kIlRec], t[kIlRec];
-            uint32_t fine[kIlRec], rr[kIlRec];
-            bool valid[kIlRec];
-#pragma unroll
-            for (int j = 0; j < kIlRec; ++j) {
-                const uint32_t bl = blk + j * (kIlThreads / 32);  // block of the round
-                const uint64_t bk = (uint64_t)b0 + k * kIlBlocksPerRound + bl;
-                rr[j] = (uint32_t)(bk * 32 + lane);
-                valid[j] = bk < (uint64_t)b0 + nblk && rr[j] >= r0 && rr[j] < r1 && !il_failed;
-                // out-of-range slots read stale bytes of the slot and are dropped below
-                const unsigned char* rec = ring + (g % kIlStages) * kSlot + bl * kBlk;
-#pragma unroll
-                for (int q2 = 0; q2 < NG; ++q2)
-                    gr[j][q2] = *reinterpret_cast<const uint2*>(rec + q2 * 256 + 8 * lane);
-                off[j] = *reinterpret_cast<const float*>(rec + 32 * kG + 4 * lane);
-                fine[j] = valid[j] ? *reinterpret_cast<const uint16_t*>(rec + 32 * kG + 128 + 2 * lane)
-                                   : 0u;
-            }
-            score_records(gr, off, fine, rr, t);
-#pragma unroll
-            for (int j = 0; j < kIlRec; ++j) {
-                // key(t, id) < tau by float compares; the key only for kept records
-                const bool keep =
-                    valid[j] && (t[j] < tau_f || (t[j] == tau_f && rr[j] < tau_id));
-                my_eval += valid[j] ? 1 : 0;
-                scan_insert(st, keys, keep, keep ? filter_key(t[j], rr[j]) : 0ull, my_pass);
-            }
-            scan_after_round<kIlThreads>(st, keys, hist, cap, kIlRound, T, tau, t_round);
-            if (il_failed) break;  // read after the barrier: the same on every thread
-            ++g_done;
-            // the slot of round g is free: thread 0 refills it with round k + kIlStages
-            const uint32_t kn = k + kIlStages;
-            if (kn < rounds) {
-                if (tid == 0)
-                    issue(g_issued, (uint64_t)b0 + kn * kIlBlocksPerRound,
-                          min(kIlBlocksPerRound, nblk - kn * kIlBlocksPerRound));
-                ++g_issued;
+        // the first cluster's first rounds go out before the table is built
+        uint32_t primed_blk0 = 0, primed_blocks = 0;
+        if (tid == 0) {
+            const uint32_t c = p.ctag[(uint64_t)qi * p.P];
+            if (c < p.C) {
+                const uint32_t r0 = p.cell_start[(uint64_t)c * F], r1 = p.cell_start[(uint64_t)c * F + F];
+                if (r1 > r0) {
+                    const uint32_t b0 = r0 >> 5, nblk = ((r1 - 1) >> 5) - b0 + 1;
+                    primed_blk0 = b0;
+                    for (uint32_t k = 0; k < (uint32_t)kIlStages && k * kIlBlocksPerRound < nblk; ++k) {
+                        const uint32_t m = min(kIlBlocksPerRound, nblk - k * kIlBlocksPerRound);
+                        issue(g_issued++, (uint64_t)b0 + k * kIlBlocksPerRound, m);
+                        primed_blocks += m;
+                    }
+                }
             }
         }
-        // realtime: the cluster's inserted records, read from the interleaved copy
-        for (uint32_t v0 = 0; v0 < ni; v0 += kIlRound) {
-            const long long t_round = clock64();
-            const uint64_t tau = st.tau;
-            uint2 gr[kIlRec][NG];
-            float off[kIlRec], t[kIlRec];
-            uint32_t fine[kIlRec], mr[kIlRec];
-            bool valid[kIlRec];
-#pragma unroll
-            for (int j = 0; j < kIlRec; ++j) {
-                const uint32_t v = v0 + tid + j * kIlThreads;
-                valid[j] = v < ni;
-                mr[j] = valid[j] ? p.ins_cl_ids[i0 + v] : 0u;
-#pragma unroll
-                for (int q2 = 0; q2 < NG; ++q2)
-                    gr[j][q2] = __ldg(reinterpret_cast<const uint2*>(
-                        p.codes_il + il_granule_offset(mr[j], q2, NSQ)));
-                off[j] = __ldg(reinterpret_cast<const float*>(p.codes_il + il_offset_offset(mr[j], NSQ)));
-                fine[j] = __ldg(reinterpret_cast<const uint16_t*>(p.codes_il + il_fine_offset(mr[j], NSQ)));
+        for (uint32_t i = tid; i < p.d; i += kIlThreads) qv[i] = p.q[(uint64_t)qi * p.d + i];
+        const float* fdk = p.fd_by_fine + (uint64_t)qi * F;
+        // the first cluster's stationary row and this query's fine terms are loaded now,
+        // so their latency overlaps the table build (srow is written after it)
+        constexpr int kPre = 2;  // float4 per thread and row (F <= kPre * 4 * kIlThreads)
+        const uint32_t c_first = p.ctag[(uint64_t)qi * p.P];
+        const bool pre = c_first < p.C && (F & 3u) == 0 && F <= kPre * 4 * kIlThreads;
+        float4 pre_st[kPre], pre_fd[kPre];
+    #pragma unroll
+        for (int u = 0; u < kPre; ++u) {
+            const uint32_t i = tid + u * kIlThreads;
+            if (pre && i < (F >> 2)) {
+                pre_st[u] = __ldg(reinterpret_cast<const float4*>(p.stationary + (uint64_t)c_first * F) + i);
+                pre_fd[u] = __ldg(reinterpret_cast<const float4*>(fdk) + i);
             }
-            score_records(gr, off, fine, mr, t);
-#pragma unroll
-            for (int j = 0; j < kIlRec; ++j) {
-                const uint64_t key = filter_key(t[j], mr[j]);
-                const bool keep = valid[j] && key < tau;
-                my_eval += valid[j] ? 1 : 0;
-                scan_insert(st, keys, keep, key, my_pass);
-            }
-            scan_after_round<kIlThreads>(st, keys, hist, cap, kIlRound, T, tau, t_round);
         }
-    }
-    if (il_failed) {
-        // a copy did not arrive in time: wait (bounded) for every copy issued, so
-        // none lands in shared memory after the block, and report the query as empty
-        for (uint32_t g = g_done; g < g_issued; ++g) il_wait(bar_of(g), (g / kIlStages) & 1u);
+        const int lut_e = HALF ? half_lut_exponent(p.qnorm[qi], p.codebook_max) : 0;
+        const float inv_scale = HALF ? ldexpf(1.0f, -lut_e) : 1.0f;
+        float4 y[NSQ / 2];
+        if (p.lsq == 4) il_load_half<NSQ>(p.codebook, tid >> 8, y);
         __syncthreads();
-        if (tid == 0) {
-            p.hcnt[qi] = 0;
-            atomicExch(p.err, 1);
+        il_build_table<NSQ, HALF, kIlThreads>(tab, stage, qv, p.codebook, p.lsq, lut_e, y);
+        unsigned long long my_eval = 0, my_pass = 0;
+        const long long t_pro = clock64();
+
+        auto score_records = [&](const uint2 (&gr)[kIlRec][NG], const float (&off)[kIlRec],
+                                 const uint32_t (&fine)[kIlRec], const uint32_t (&mr)[kIlRec],
+                                 float (&t)[kIlRec]) {
+            il_score<NSQ, HALF, kIlRec>(tab, srow, gr, off, fine, mr, inv_scale, t);
+        };
+
+        for (uint32_t l = 0; l < p.P && !il_failed; ++l) {
+            if (!scan_cluster_begin(p, st, qi, l)) break;  // (its first barrier ends the table)
+            const uint32_t r0 = st.r0, r1 = st.r1, i0 = st.i0, ni = st.i1 - st.i0;
+            if (r1 - r0 + ni == 0) continue;
+            if (tid == 0) st.n_records += r1 - r0 + ni;
+            if (l == 0 && pre) {
+                // srow from the rows loaded before the table build
+                const float cdl = st.cdl;
+                float4* s4 = reinterpret_cast<float4*>(srow);
+    #pragma unroll
+                for (int u = 0; u < kPre; ++u) {
+                    const uint32_t i = tid + u * kIlThreads;
+                    if (i < (F >> 2)) {
+                        const float4 a = pre_st[u], b = pre_fd[u];
+                        s4[i] = make_float4(2.0f * __fadd_rn(__fadd_rn(cdl, a.x), b.x),
+                                            2.0f * __fadd_rn(__fadd_rn(cdl, a.y), b.y),
+                                            2.0f * __fadd_rn(__fadd_rn(cdl, a.z), b.z),
+                                            2.0f * __fadd_rn(__fadd_rn(cdl, a.w), b.w));
+                    }
+                }
+                __syncthreads();
+            } else {
+                scan_fill_srow(p, srow, fdk, st.c, st.cdl);
+            }
+            uint32_t b0 = 0, nblk = 0, rounds = 0;
+            if (r1 > r0) {
+                b0 = r0 >> 5;
+                nblk = ((r1 - 1) >> 5) - b0 + 1;
+                rounds = (nblk + kIlBlocksPerRound - 1) / kIlBlocksPerRound;
+            }
+            // rounds of this cluster already in flight (the first cluster's, primed)
+            uint32_t sent = (l == 0 && primed_blocks > 0 && primed_blk0 == b0)
+                                ? (primed_blocks + kIlBlocksPerRound - 1) / kIlBlocksPerRound
+                                : 0;
+            if (tid == 0) {
+                for (; sent < rounds && sent < (uint32_t)kIlStages; ++sent)
+                    issue(g_issued++, (uint64_t)b0 + sent * kIlBlocksPerRound,
+                          min(kIlBlocksPerRound, nblk - sent * kIlBlocksPerRound));
+            }
+            sent = rounds < (uint32_t)kIlStages ? rounds : (uint32_t)kIlStages;
+            g_issued = g_done + sent;  // every thread tracks the count thread 0 issued
+            const uint32_t blk = tid >> 5, lane = tid & 31;
+            for (uint32_t k = 0; k < rounds; ++k) {
+                const long long t_round = clock64();
+                const uint64_t tau = st.tau;
+                // tau as (float, id): key(t, id) < tau iff t < tau_f, or t == tau_f and
+                // id < tau_id (float compares treat -0 as +0, as the keys do; a bound
+                // whose float part is the key of -0 keeps exactly the t < 0)
+                float tau_f = tau == kKeyMax ? __int_as_float(0x7f800000) : key_value(tau);
+                uint32_t tau_id = tau == kKeyMax ? 0xFFFFFFFFu : (uint32_t)tau;
+                if ((uint32_t)(tau >> 32) == 0x7FFFFFFFu) {
+                    tau_f = 0.0f;
+                    tau_id = 0;
+                }
+                const uint32_t g = g_done;
+                if (!il_wait(bar_of(g), (g / kIlStages) & 1u)) {
+                    if (lane == 0) atomicExch(&il_failed, 1);
+                }
+                uint2 gr[kIlRec][NG];
+                float off[kIlRec], t[kIlRec];
+                uint32_t fine[kIlRec], rr[kIlRec];
+                bool valid[kIlRec];
+    #pragma unroll
+                for (int j = 0; j < kIlRec; ++j) {
+                    const uint32_t bl = blk + j * (kIlThreads / 32);  // block of the round
+                    const uint64_t bk = (uint64_t)b0 + k * kIlBlocksPerRound + bl;
+                    rr[j] = (uint32_t)(bk * 32 + lane);
+                    valid[j] = bk < (uint64_t)b0 + nblk && rr[j] >= r0 && rr[j] < r1 && !il_failed;
+                    // out-of-range slots read stale bytes of the slot and are dropped below
+                    const unsigned char* rec = ring + (g % kIlStages) * kSlot + bl * kBlk;
+    #pragma unroll
+                    for (int q2 = 0; q2 < NG; ++q2)
+                        gr[j][q2] = *reinterpret_cast<const uint2*>(rec + q2 * 256 + 8 * lane);
+                    off[j] = *reinterpret_cast<const float*>(rec + 32 * kG + 4 * lane);
+                    fine[j] = valid[j] ? *reinterpret_cast<const uint16_t*>(rec + 32 * kG + 128 + 2 * lane)
+                                       : 0u;
+                }
+                score_records(gr, off, fine, rr, t);
+    #pragma unroll
+                for (int j = 0; j < kIlRec; ++j) {
+                    // key(t, id) < tau by float compares; the key only for kept records
+                    const bool keep =
+                        valid[j] && (t[j] < tau_f || (t[j] == tau_f && rr[j] < tau_id));
+                    my_eval += valid[j] ? 1 : 0;
+                    scan_insert(st, keys, keep, keep ? filter_key(t[j], rr[j]) : 0ull, my_pass);
+                }
+                scan_after_round<kIlThreads>(st, keys, hist, cap, kIlRound, T, tau, t_round);
+                if (il_failed) break;  // read after the barrier: the same on every thread
+                ++g_done;
+                // the slot of round g is free: thread 0 refills it with round k + kIlStages
+                const uint32_t kn = k + kIlStages;
+                if (kn < rounds) {
+                    if (tid == 0)
+                        issue(g_issued, (uint64_t)b0 + kn * kIlBlocksPerRound,
+                              min(kIlBlocksPerRound, nblk - kn * kIlBlocksPerRound));
+                    ++g_issued;
+                }
+            }
+            // realtime: the cluster's inserted records, read from the interleaved copy
+            for (uint32_t v0 = 0; v0 < ni; v0 += kIlRound) {
+                const long long t_round = clock64();
+                const uint64_t tau = st.tau;
+                uint2 gr[kIlRec][NG];
+                float off[kIlRec], t[kIlRec];
+                uint32_t fine[kIlRec], mr[kIlRec];
+                bool valid[kIlRec];
+    #pragma unroll
+                for (int j = 0; j < kIlRec; ++j) {
+                    const uint32_t v = v0 + tid + j * kIlThreads;
+                    valid[j] = v < ni;
+                    mr[j] = valid[j] ? p.ins_cl_ids[i0 + v] : 0u;
+    #pragma unroll
+                    for (int q2 = 0; q2 < NG; ++q2)
+                        gr[j][q2] = __ldg(reinterpret_cast<const uint2*>(
+                            p.codes_il + il_granule_offset(mr[j], q2, NSQ)));
+                    off[j] = __ldg(reinterpret_cast<const float*>(p.codes_il + il_offset_offset(mr[j], NSQ)));
+                    fine[j] = __ldg(reinterpret_cast<const uint16_t*>(p.codes_il + il_fine_offset(mr[j], NSQ)));
+                }
+                score_records(gr, off, fine, mr, t);
+    #pragma unroll
+                for (int j = 0; j < kIlRec; ++j) {
+                    const uint64_t key = filter_key(t[j], mr[j]);
+                    const bool keep = valid[j] && key < tau;
+                    my_eval += valid[j] ? 1 : 0;
+                    scan_insert(st, keys, keep, key, my_pass);
+                }
+                scan_after_round<kIlThreads>(st, keys, hist, cap, kIlRound, T, tau, t_round);
+            }
         }
-        return;
+        if (il_failed) {
+            // a copy did not arrive in time: wait (bounded) for every copy issued, so
+            // none lands in shared memory after the block, and report the query as empty
+            for (uint32_t g = g_done; g < g_issued; ++g) il_wait(bar_of(g), (g / kIlStages) & 1u);
+            __syncthreads();
+            if (tid == 0) {
+                p.hcnt[qi] = 0;
+                atomicExch(p.err, 1);
+            }
+            return;
+        }
+        scan_finish<kIlThreads>(p, st, keys, hist, qi, my_eval, my_eval, my_pass, t_start, t_pro);
     }
-    scan_finish<kIlThreads>(p, st, keys, hist, qi, my_eval, my_eval, my_pass, t_start, t_pro);
 }
 
 // Launch order of the scan's blocks. A block's time follows the records of the
 // clusters its query probes, and blocks start in index order: queries sorted by
 // descending record count start the longest scans first and end the grid with the
 // shortest, so fewer SMs sit idle at the tail. The sort is by bucket (4 steps per
-// octave of the count), which is all the ordering needs; the results do not depend
-// on it.
-constexpr uint32_t kOrderBuckets = 132;
+// octave of the count), which is all that needs; within a bucket by the first probed
+// cluster, in kOrderGroups groups of clusters, so that queries of one cluster run at
+// about the same time and find its records, and the rerank its vectors, in L2. The
+// results do not depend on it.
+constexpr uint32_t kOrderBuckets = 132, kOrderGroups = 62;
+constexpr uint32_t kOrderBins = kOrderBuckets * kOrderGroups;
 constexpr int kOrderThreads = 1024;
-
+constexpr uint32_t kOrderPer = (kOrderBins + kOrderThreads - 1) / kOrderThreads;
 __device__ __forceinline__ uint32_t work_bucket(uint32_t w) {
     if (w == 0) return kOrderBuckets - 1;  // nothing to scan: last
     const int e = 31 - __clz(w);
@@ -1259,89 +1292,126 @@ __device__ __forceinline__ uint32_t work_bucket(uint32_t w) {
     return (kOrderBuckets - 2) - ((uint32_t)e * 4 + frac);  // more records: earlier
 }
 
-// One thread per query: its record count over the probed clusters, as a bucket.
+// One thread per query: its record count over the probed clusters, as a bin.
 __global__ void k_scan_work(const uint32_t* __restrict__ ctag, const int32_t* __restrict__ status,
                             const uint32_t* __restrict__ cell_start,
                             const uint32_t* __restrict__ ins_cl_start, uint32_t n, uint32_t P,
-                            uint32_t C, uint32_t F, uint8_t* __restrict__ wbucket) {
+                            uint32_t C, uint32_t F, uint16_t* __restrict__ wbin) {
     const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= n) return;
-    uint32_t w = 0;
+    uint32_t w = 0, first = 0;
     if (status[q] == 0) {
         for (uint32_t l = 0; l < P; ++l) {
             const uint32_t c = ctag[(uint64_t)q * P + l];
             if (c >= C) break;  // the probed clusters fill a prefix of the slots
+            if (l == 0) first = (uint32_t)((uint64_t)c * kOrderGroups / C);
             w += cell_start[(uint64_t)c * F + F] - cell_start[(uint64_t)c * F];
             if (ins_cl_start) w += ins_cl_start[c + 1] - ins_cl_start[c];
         }
     }
-    wbucket[q] = (uint8_t)work_bucket(w);
+    wbin[q] = (uint16_t)(work_bucket(w) * kOrderGroups + first);
 }
 
-// One block: counting sort of the queries by bucket (order within a bucket is free).
-__global__ __launch_bounds__(kOrderThreads) void k_scan_order(const uint8_t* __restrict__ wbucket,
-                                                              uint32_t n, uint32_t* __restrict__ order) {
-    __shared__ uint32_t hist[kOrderBuckets];
-    for (uint32_t i = threadIdx.x; i < kOrderBuckets; i += kOrderThreads) hist[i] = 0;
+// One block: counting sort of the queries by bin (order within a bin is free). The
+// count of queries left to the fused scan starts at 0.
+__global__ __launch_bounds__(kOrderThreads) void k_scan_order(const uint16_t* __restrict__ wbin,
+                                                              uint32_t n, uint32_t* __restrict__ order,
+                                                              uint32_t* __restrict__ ntodo) {
+    __shared__ uint32_t hist[kOrderPer * kOrderThreads];
+    __shared__ uint32_t wsum[kOrderThreads / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) *ntodo = 0;
+    for (uint32_t i = tid; i < kOrderPer * kOrderThreads; i += kOrderThreads) hist[i] = 0;
     __syncthreads();
-    for (uint32_t q = threadIdx.x; q < n; q += kOrderThreads) atomicAdd(&hist[wbucket[q]], 1u);
+    for (uint32_t q = tid; q < n; q += kOrderThreads) atomicAdd(&hist[wbin[q]], 1u);
     __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t run = 0;
-        for (uint32_t i = 0; i < kOrderBuckets; ++i) {
-            const uint32_t c = hist[i];
-            hist[i] = run;
-            run += c;
-        }
+    uint32_t c[kOrderPer], run = 0;
+#pragma unroll
+    for (uint32_t j = 0; j < kOrderPer; ++j) {
+        c[j] = hist[tid * kOrderPer + j];
+        run += c[j];
+    }
+    uint32_t incl = run;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    if (lane == 31) wsum[warp] = incl;
+    __syncthreads();
+    uint32_t at = incl - run;
+    for (int w = 0; w < warp; ++w) at += wsum[w];
+#pragma unroll
+    for (uint32_t j = 0; j < kOrderPer; ++j) {
+        hist[tid * kOrderPer + j] = at;
+        at += c[j];
     }
     __syncthreads();
-    for (uint32_t q = threadIdx.x; q < n; q += kOrderThreads)
-        order[atomicAdd(&hist[wbucket[q]], 1u)] = q;
+    for (uint32_t q = tid; q < n; q += kOrderThreads) order[atomicAdd(&hist[wbin[q]], 1u)] = q;
 }
 
 // ------------------------------------------------------------ split scan
-// The interleaved layout's scan when the per-pass scratch holds the distance of every
-// record the batch scans (Scratch::tbuf); queries that do not fit, or whose cut bin
-// holds too many records, stay with k_scan_il. One block per query (k_scan_score):
-//   1. the table (il_build_table), then, per probed cluster, the cell terms;
-//   2. the histogram's range from one record per thread at evenly spaced positions of
-//      the first probed cluster;
-//   3. records, with no barrier: each warp streams its own record blocks straight
-//      from the interleaved copy (coalesced 8-byte loads, the next step's loads in
-//      flight while the current one is scored), writes each record's t (the same
-//      il_score arithmetic as k_scan_il) to tbuf, query q's records at qoff[q] cluster
-//      by cluster (base records, then inserted ones), and counts it in a
-//      kSplitBins-bin histogram linear in t;
-//   4. the cut: the bin where the running count reaches T; every record of a higher
-//      bin has T records strictly below it;
-//   5. the pick: the block reads its own distances back (mostly from L2), keeps those
-//      at or below the cut bin as (t, position) keys in the table's place, maps
-//      positions to memory ids and writes the exact T smallest (t, id), unordered:
-//      the same set as k_scan_il's.
-// Without k_scan_il's key buffer and its cut-backs, a block holds the table, the cell
-// terms and the histogram: two blocks per SM, so one block's table build and pick
-// overlap the other's records. The FP16 table (precision form) keeps one entry per
-// 4-byte slot, the FP32 table's addresses: a lookup is the same PRMT, load and add
+// The interleaved layout's scan. One block per query (k_scan_score), two blocks per SM:
+//   1. the probed clusters' record ranges and the table (il_build_table);
+//   2. a bound on the T-th smallest distance, when the query has more records than the
+//      key buffer takes: the r-th smallest t of S records at evenly spaced positions,
+//      r far enough above its expectation S T / N that fewer than T records at or below
+//      it are improbable (sample_rank);
+//   3. records, with no barrier: the clusters go through in groups whose cell terms fit
+//      shared memory together; each warp streams its own record blocks of the group
+//      straight from the interleaved copy (coalesced 8-byte loads, the next step's loads
+//      in flight while the current one is scored, the same il_score arithmetic as
+//      k_scan_il) and appends the (t, id) keys at or below the bound to the buffer, one
+//      shared atomic per warp and step;
+//   4. the exact T smallest keys of the buffer, written unordered: the same set as
+//      k_scan_il's, since every record left out lies above T others.
+// A query whose buffer overflowed, or got fewer than T keys, goes to k_scan_il's list:
+// the bound only decides who answers. The FP16 table (precision form) keeps one entry
+// per 4-byte slot, the FP32 table's addresses: a lookup is the same PRMT, load and add
 // (the compact 2-byte layout costs a shift per lookup, and its smaller footprint buys
 // nothing here).
-// record blocks per warp and step (FP32 table, FP16 table)
-#ifndef PGPU_SPLIT_RB32
-#define PGPU_SPLIT_RB32 4
-#endif
-#ifndef PGPU_SPLIT_RB16
-#define PGPU_SPLIT_RB16 4
+//
+// Bound by instruction issue: per record 24 (nsq) lookups of three instructions, and one
+// 128-byte shared-memory wavefront each. With two blocks
+// per SM one block's table and bound overlap the other's records only in part (a block
+// alone does not fill the SM): of a block's 50k SM cycles in 10k queries over 28.8k records
+// of 24 codes each, 33k are the records'. That batch takes 1.63 ms; 2.09 with every
+// distance written out, binned and read back, and 25 us more for the record counts and the
+// fused kernel's idle blocks.
+#ifndef PGPU_SPLIT_REC
+#define PGPU_SPLIT_REC 4
 #endif
 constexpr int kSplitThreads = 256;
 constexpr int kSplitWarps = kSplitThreads / 32;
-constexpr uint32_t kSplitBins = 4096;
-constexpr uint32_t kSplitMaxSlots = 512;   // probed clusters a split query may have
-constexpr uint32_t kSplitNo = 0xFFFFFFFFu; // count of a query left to k_scan_il
-#ifndef PGPU_SPLIT_AHEAD
-#define PGPU_SPLIT_AHEAD 2
-#endif
-constexpr int kSplitAhead = PGPU_SPLIT_AHEAD;  // L2 prefetch distance in record steps (-1: none)
-// candidates the pick phase holds (in the table's place): 8192
-__host__ __device__ constexpr uint32_t split_max_keys(bool) { return il_table_bytes(false) / 8; }
+constexpr int kSplitRec = PGPU_SPLIT_REC;    // record blocks per warp and step (il_bytes)
+static_assert(kSplitRec <= 4, "il_bytes has room for steps of 4 blocks");
+constexpr uint32_t kSplitMaxSlots = 512;     // probed clusters a split query may have
+constexpr uint32_t kSplitRows = 4096;        // floats of cell terms a group of clusters may take
+
+// Shared memory: table, query, slot arrays, cell terms, then the keys (the compact table
+// while the table is built, before them the sampled keys and their select's histogram).
+struct SplitLayout {
+    uint32_t slots, rows_per, group, srow, keys, cap, bytes;
+};
+__host__ __device__ inline SplitLayout split_layout(uint32_t nsq, uint32_t d, uint32_t F, uint32_t P,
+                                                    uint32_t budget) {
+    SplitLayout y;
+    const uint32_t maxl = P < kSplitMaxSlots ? P : kSplitMaxSlots;
+    y.slots = il_table_bytes(false) + il_query_bytes(d);
+    y.rows_per = (F + 3u) & ~3u;
+    y.group = kSplitRows / y.rows_per;
+    y.group = y.group < 1 ? 1 : (y.group > maxl ? maxl : y.group);
+    y.srow = y.slots + (6u * 4u * (maxl + 1) + 15u) / 16u * 16u;
+    y.keys = y.srow + y.group * y.rows_per * 4u;
+    const uint32_t stage = (nsq * 257u * 4u + 7u) & ~7u;
+    const uint32_t room = budget > y.keys ? budget - y.keys : 0u;
+    y.cap = room / 8u;
+    y.bytes = room >= stage ? y.keys + y.cap * 8u : 0u;
+    return y;
+}
+// Two blocks per SM when the buffer then takes T keys one and a half times over, else one.
+constexpr uint32_t kSplitBudget2 = 111 * 1024, kSplitBudget1 = 220 * 1024;
+__host__ __device__ inline uint32_t split_need(uint32_t T) { return T + T / 2 + 512; }
 
 struct SplitParams {
     const uint32_t* ctag;
@@ -1357,522 +1427,464 @@ struct SplitParams {
     const float* codebook;
     const uint8_t* codes_il;
     const uint32_t* order;
-    uint32_t* qcnt;
-    uint32_t* qoff;
-    uint32_t* qflag;
-    SplitCut* cut;
-    float* tbuf;
+    uint32_t* todo;                // queries left to k_scan_il, and their number
+    uint32_t* ntodo;
     float* hdist;
     uint32_t* htag;
     uint32_t* hcnt;
     unsigned long long* counters;
-    uint64_t tcap;  // floats tbuf holds
     uint32_t n, d, C, F, lsq, P, T;
     float codebook_max;
+    SplitLayout lay;
 };
 
-// bin(t) = clamp(trunc((t - lo) * scale), 0, kSplitBins - 1): non-decreasing in t
-// (each step rounds monotonically; a NaN product, 0 * inf at t = lo, converts to 0).
-__device__ __forceinline__ uint32_t split_bin(float t, float lo, float scale) {
-    const int b = __float2int_rz(__fmul_rn(__fsub_rn(t, lo), scale));
-    return (uint32_t)min(max(b, 0), (int)kSplitBins - 1);
-}
-
-// One thread per query: records over its probed clusters (kSplitNo: not split).
-__global__ void k_split_counts(SplitParams sp) {
-    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= sp.n) return;
-    uint32_t w = kSplitNo;
-    if (sp.status[q] == 0) {
-        w = 0;
-        for (uint32_t l = 0; l < sp.P; ++l) {
-            const uint32_t c = sp.ctag[(uint64_t)q * sp.P + l];
-            if (c >= sp.C) break;  // the probed clusters fill a prefix of the slots
-            if (l >= kSplitMaxSlots) {
-                w = kSplitNo;
-                break;
-            }
-            w += sp.cell_start[(uint64_t)c * sp.F + sp.F] - sp.cell_start[(uint64_t)c * sp.F];
-            if (sp.ins_cl_start) w += sp.ins_cl_start[c + 1] - sp.ins_cl_start[c];
-        }
-    }
-    sp.qcnt[q] = w;
-}
-
-// One block: each query's place in tbuf (its records rounded up to 4 floats, so
-// every query starts 16-byte aligned), in query order; a query fits when its records
-// end within tcap, and only fitting queries are flagged for the split scan.
-__global__ __launch_bounds__(1024) void k_split_offsets(SplitParams sp) {
-    __shared__ unsigned long long wsum[32];
-    __shared__ unsigned long long base;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) base = 0;
-    __syncthreads();
-    for (uint32_t q0 = 0; q0 < sp.n; q0 += 1024) {
-        const uint32_t q = q0 + threadIdx.x;
-        const uint32_t w = q < sp.n ? sp.qcnt[q] : kSplitNo;
-        const unsigned long long v = w == kSplitNo ? 0ull : ((unsigned long long)w + 3) & ~3ull;
-        const unsigned long long b0 = base;
-        unsigned long long x = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
-        }
-        if (lane == 31) wsum[warp] = x;
-        __syncthreads();
-        if (warp == 0) {
-            unsigned long long z = wsum[lane];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const unsigned long long y = __shfl_up_sync(0xffffffffu, z, o);
-                if (lane >= o) z += y;
-            }
-            wsum[lane] = z;
-        }
-        __syncthreads();
-        const unsigned long long excl = b0 + (warp ? wsum[warp - 1] : 0ull) + x - v;
-        if (q < sp.n) {
-            const bool fits = w != kSplitNo && excl + v <= sp.tcap;
-            sp.qoff[q] = fits ? (uint32_t)excl : 0u;
-            sp.qflag[q] = fits ? 1u : 0u;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) base = b0 + wsum[31];
-        __syncthreads();
-    }
+// 1-based rank, among S evenly spaced records of N, of the bound for the T smallest: the
+// expected rank S T / N, three and a half standard deviations (four neighbours are sampled
+// together, and neighbours are alike: 2.5 times the variance of independent ones) and three.
+__device__ __forceinline__ uint32_t sample_rank(uint32_t S, uint32_t T, uint32_t N) {
+    const float e = (float)S * (float)T / (float)N;
+    return (uint32_t)(e + 3.5f * sqrtf(2.5f * e) + 3.0f);
 }
 
 template <int NSQ, bool HALF>
-#ifndef PGPU_SPLIT_MINB16
-#define PGPU_SPLIT_MINB16 2
-#endif
-__global__ __launch_bounds__(kSplitThreads, HALF ? PGPU_SPLIT_MINB16 : 2) void k_scan_score(SplitParams sp) {
+__global__ __launch_bounds__(kSplitThreads, 2) void k_scan_score(const __grid_constant__ SplitParams sp) {
     constexpr int NG = (NSQ + 7) / 8;  // 8-byte code granules per record
     constexpr uint32_t kG = NG * 8;
     constexpr uint32_t kBlk = 32 * kG + 192;  // il_block_bytes
-    constexpr int NW = kSplitWarps, RB = HALF ? PGPU_SPLIT_RB16 : PGPU_SPLIT_RB32;
+    constexpr int NW = kSplitWarps, RB = kSplitRec, NT = kSplitThreads;
     extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ uint32_t s_c, s_r0, s_r1, s_i0, s_i1;
-    __shared__ float s_cdl;
-    __shared__ float s_lo[NW], s_hi[NW];
-    __shared__ uint32_t s_red[NW], s_bin;
-    // the pick phase's select scratch (block_kth_hist) and counters
-    __shared__ uint32_t k_red[2 * NW + 2], k_hist256[256], k_cnt, k_count, k_slots, k_out;
+    __shared__ uint32_t s_red[NW];
+    // select scratch (block_kth_hist) and counters
+    __shared__ uint32_t k_red[2 * NW + 2], k_hist256[256], k_cnt, k_count, k_out;
     __shared__ uint64_t k_sel[4];
     const uint32_t qi = sp.order[blockIdx.x];
-    if (!sp.qflag[qi]) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t F = sp.F, T = sp.T;
+    const uint32_t F = sp.F, T = sp.T, cap = sp.lay.cap, Fp = sp.lay.rows_per;
+    float4 y[NSQ / 2];
+    if (sp.lsq == 4) il_load_half<NSQ>(sp.codebook, 0, y);
+    if (sp.status[qi] != 0) {
+        if (tid == 0) sp.hcnt[qi] = 0;
+        return;
+    }
+    // more probed clusters than slots: the fused kernel's
+    if (sp.P > kSplitMaxSlots && sp.ctag[(uint64_t)qi * sp.P + kSplitMaxSlots] < sp.C) {
+        if (tid == 0) sp.todo[atomicAdd(sp.ntodo, 1u)] = qi;
+        return;
+    }
     unsigned char* tab = smem;
-    // the FP16 table takes one 4-byte slot per entry (the FP32 table's addresses and size)
     float* qv = reinterpret_cast<float*>(smem + il_table_bytes(false));
-    unsigned char* rest = smem + il_table_bytes(false) + il_query_bytes(sp.d);
-    float* stage = reinterpret_cast<float*>(rest);  // [NSQ][257] while the table is built
-    float* srow = reinterpret_cast<float*>(rest);   // [F] afterwards
-    uint32_t* hist = reinterpret_cast<uint32_t*>(rest + il_srow_bytes(F));  // [kSplitBins]
-    // the probed clusters' record positions: start, base records, first memory id,
-    // first inserted slot
-    uint32_t* sl_start = hist + kSplitBins;  // [kSplitMaxSlots + 1]
-    uint32_t* sl_nb = sl_start + kSplitMaxSlots + 1;
-    uint32_t* sl_r0 = sl_nb + kSplitMaxSlots;
-    uint32_t* sl_i0 = sl_r0 + kSplitMaxSlots;
-    for (uint32_t i = tid; i < sp.d; i += kSplitThreads) qv[i] = sp.q[(uint64_t)qi * sp.d + i];
+    const uint32_t maxl = sp.P < kSplitMaxSlots ? sp.P : kSplitMaxSlots;
+    // per probed cluster: first record position of the query's (one past the last at [L]),
+    // base records, first memory id, first inserted slot, id, distance
+    uint32_t* sl_start = reinterpret_cast<uint32_t*>(smem + sp.lay.slots);
+    uint32_t* sl_nb = sl_start + maxl + 1;
+    uint32_t* sl_r0 = sl_nb + maxl + 1;
+    uint32_t* sl_i0 = sl_r0 + maxl + 1;
+    uint32_t* sl_c = sl_i0 + maxl + 1;
+    float* sl_cd = reinterpret_cast<float*>(sl_c + maxl + 1);
+    float* srow = reinterpret_cast<float*>(smem + sp.lay.srow);      // [group][Fp] cell terms
+    uint64_t* keys = reinterpret_cast<uint64_t*>(smem + sp.lay.keys);  // [cap]
+    float* stage = reinterpret_cast<float*>(keys);                   // [NSQ][257] before
+    for (uint32_t i = tid; i < sp.d; i += NT) qv[i] = sp.q[(uint64_t)qi * sp.d + i];
     const int lut_e = HALF ? half_lut_exponent(sp.qnorm[qi], sp.codebook_max) : 0;
     const float inv_scale = HALF ? ldexpf(1.0f, -lut_e) : 1.0f;
-    __syncthreads();
-    il_build_table<NSQ, HALF, kSplitThreads, true>(tab, stage, qv, sp.codebook, sp.lsq, lut_e);
-    __syncthreads();  // stage (under srow and hist) is read to the end of the expansion
-    for (uint32_t b = tid; b < kSplitBins; b += kSplitThreads) hist[b] = 0;
-    // slot table: records per probed cluster, then an exclusive scan (PS slots per thread)
-    const uint32_t maxl = sp.P < kSplitMaxSlots ? sp.P : kSplitMaxSlots;
     if (tid == 0) {
         k_count = 0;
         k_out = 0;
-        k_slots = maxl;
+        k_cnt = 0;
     }
-    __syncthreads();
-    for (uint32_t l = tid; l < maxl; l += kSplitThreads)
-        if (sp.ctag[(uint64_t)qi * sp.P + l] >= sp.C) atomicMin(&k_slots, l);
-    __syncthreads();
-    const uint32_t L = k_slots;
-    {
-        constexpr int PS = kSplitMaxSlots / kSplitThreads;
-        uint32_t len[PS], run = 0;
+    // slot table: PS slots per thread, then an exclusive scan of the records
+    constexpr int PS = (int)kSplitMaxSlots / NT;
+    static_assert(PS * NT == (int)kSplitMaxSlots, "slots split evenly over the threads");
+    uint32_t len[PS], c[PS], run = 0, L = 0;
 #pragma unroll
-        for (int j = 0; j < PS; ++j) {
-            const uint32_t l = tid * PS + j;
-            len[j] = 0;
-            if (l < L) {
-                const uint32_t c = sp.ctag[(uint64_t)qi * sp.P + l];
-                const uint32_t r0 = sp.cell_start[(uint64_t)c * F], r1 = sp.cell_start[(uint64_t)c * F + F];
-                uint32_t i0 = 0, i1 = 0;
-                if (sp.ins_cl_start) {
-                    i0 = sp.ins_cl_start[c];
-                    i1 = sp.ins_cl_start[c + 1];
-                }
-                sl_nb[l] = r1 - r0;
-                sl_r0[l] = r0;
-                sl_i0[l] = i0;
-                len[j] = (r1 - r0) + (i1 - i0);
+    for (int j = 0; j < PS; ++j) {
+        const uint32_t l = tid * PS + j;
+        c[j] = l < maxl ? sp.ctag[(uint64_t)qi * sp.P + l] : sp.C;
+    }
+#pragma unroll
+    for (int j = 0; j < PS; ++j) {
+        const uint32_t l = tid * PS + j;
+        len[j] = 0;
+        if (c[j] < sp.C) {
+            const uint32_t* cell0 = sp.cell_start + (uint64_t)c[j] * F;
+            const uint32_t r0 = cell0[0], r1 = cell0[F];
+            uint32_t i0 = 0, i1 = 0;
+            if (sp.ins_cl_start) {
+                i0 = sp.ins_cl_start[c[j]];
+                i1 = sp.ins_cl_start[c[j] + 1];
             }
-            run += len[j];
+            sl_c[l] = c[j];
+            sl_cd[l] = sp.cdist[(uint64_t)qi * sp.P + l];
+            sl_nb[l] = r1 - r0;
+            sl_r0[l] = r0;
+            sl_i0[l] = i0;
+            len[j] = (r1 - r0) + (i1 - i0);
         }
-        uint32_t incl = run;
+        run += len[j];
+    }
+    // the probed clusters fill a prefix of the slots
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += y;
+    for (int j = 0; j < PS; ++j) L += (uint32_t)__syncthreads_count(c[j] < sp.C);
+    uint32_t incl = run;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    if (lane == 31) s_red[warp] = incl;
+    const float* fdk = sp.fd_by_fine + (uint64_t)qi * F;
+    // cell terms of slots [l0, l1): srow[f] = 2 * cell_dist of cell f, cell_dist =
+    // (cd + stationary) + fd (puck_index.cpp:539-540)
+    auto fill_rows = [&](uint32_t l0, uint32_t l1) {
+        if ((F & 3u) == 0) {
+            const uint32_t w4 = ((F >> 2) + 31u) & ~31u;  // a warp stays within a row
+#pragma unroll 4
+            for (uint32_t e = tid; e < (l1 - l0) * w4; e += NT) {
+                const uint32_t l = e / w4, i = e - l * w4;
+                if (i < (F >> 2)) {
+                    const float cdl = sl_cd[l0 + l];
+                    const float4 a =
+                        __ldg(reinterpret_cast<const float4*>(sp.stationary + (uint64_t)sl_c[l0 + l] * F) + i);
+                    const float4 b = __ldg(reinterpret_cast<const float4*>(fdk) + i);
+                    reinterpret_cast<float4*>(srow + l * Fp)[i] =
+                        make_float4(2.0f * __fadd_rn(__fadd_rn(cdl, a.x), b.x),
+                                    2.0f * __fadd_rn(__fadd_rn(cdl, a.y), b.y),
+                                    2.0f * __fadd_rn(__fadd_rn(cdl, a.z), b.z),
+                                    2.0f * __fadd_rn(__fadd_rn(cdl, a.w), b.w));
+                }
+            }
+        } else {
+            for (uint32_t l = l0; l < l1; ++l)
+                for (uint32_t i = tid; i < F; i += NT)
+                    srow[(l - l0) * Fp + i] =
+                        2.0f * __fadd_rn(__fadd_rn(sl_cd[l], sp.stationary[(uint64_t)sl_c[l] * F + i]), fdk[i]);
         }
-        if (lane == 31) s_red[warp] = incl;
-        __syncthreads();
+    };
+    fill_rows(0, min(sp.lay.group, L));
+    il_build_table<NSQ, HALF, NT, true>(tab, stage, qv, sp.codebook, sp.lsq, lut_e, y);
+    // (its barrier also ends the writes of s_red)
+    {
         uint32_t st0 = incl - run;
         for (int w = 0; w < warp; ++w) st0 += s_red[w];
 #pragma unroll
         for (int j = 0; j < PS; ++j) {
             const uint32_t l = tid * PS + j;
-            if (l < L) sl_start[l] = st0;
+            if (l < L) {
+                sl_start[l] = st0;
+                if (l == L - 1) sl_start[L] = st0 + len[j];
+            }
             st0 += len[j];
         }
-        if (tid == kSplitThreads - 1) sl_start[L] = st0;  // the total
+        if (L == 0 && tid == 0) sl_start[0] = 0;
     }
     __syncthreads();
     const uint32_t N = sl_start[L];  // records of all probed clusters
-    // slot of record position ps (the last slot starting at or before it)
-    auto slot_of = [&](uint32_t ps) {
-        uint32_t a = 0, b = L;
-        while (b - a > 1) {
-            const uint32_t mid = (a + b) >> 1;
-            if (sl_start[mid] <= ps) a = mid;
-            else b = mid;
+    float tau = __int_as_float(0x7f800000);
+    if (N > cap) {
+        // the bound, from S sampled records: as many as it takes for the candidates expected
+        // to fit, four or two per thread at a time. Four neighbouring lanes take the records of their
+        // own lanes in one record block: whole sectors, and lookups without bank conflicts.
+        uint32_t S = 2 * NT;
+        while (S + 2 * NT + kHistBins / 2 <= cap) {
+            const float r = (float)sample_rank(S, T, N), per = (float)N / (float)S;
+            if (r * per + 3.0f * sqrtf(r) * per <= 0.9f * (float)cap && S * 96 >= N) break;
+            S += 2 * NT;
         }
-        return a;
-    };
-    float* out = sp.tbuf + sp.qoff[qi];
-    const float* fdk = sp.fd_by_fine + (uint64_t)qi * F;
-    uint32_t pos = 0;  // records written (the same on every thread)
-    float lo = 0.0f, scale = 0.0f;
-    // the histogram's range: the smallest and largest of one t per thread (ok: the
-    // thread has one). All threads; barrier inside.
-    auto set_range = [&](float t1, bool ok) {
-        float mn = ok ? t1 : __int_as_float(0x7f800000), mx = ok ? t1 : __int_as_float(0xff800000);
+        const float step = (float)N / (float)S;
+        auto sample = [&](uint32_t i0, auto count) {
+            constexpr int R = decltype(count)::value;
+            uint32_t m[R], f[R];
+            uint2 g[R][NG];
+            float o[R], t[R], cterm[R];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        }
-        if (lane == 0) {
-            s_lo[warp] = mn;
-            s_hi[warp] = mx;
-        }
-        __syncthreads();
-        mn = s_lo[0];
-        mx = s_hi[0];
-#pragma unroll
-        for (int w = 1; w < NW; ++w) {
-            mn = fminf(mn, s_lo[w]);
-            mx = fmaxf(mx, s_hi[w]);
-        }
-        if (mx > mn) {
-            lo = mn;
-            scale = __fdiv_rn((float)(kSplitBins - 1), __fsub_rn(mx, mn));
-        } else {
-            lo = mn > -3.0e38f && mn < 3.0e38f ? mn : 0.0f;
-            scale = 0.0f;
-        }
-    };
-    {
-        // the histogram's range: t of one record per thread at evenly spaced positions
-        // of all probed clusters (its cell term read from global memory; the range only
-        // has to be the same for every record, not exact)
-        const bool ok = N > 0;
-        const uint32_t ps = ok ? (uint32_t)(((uint64_t)tid * N) / kSplitThreads) : 0u;
-        const uint32_t a = ok ? slot_of(ps) : 0u;
-        const uint32_t local = ps - sl_start[a];
-        uint32_t m1[1];
-        m1[0] = !ok ? 0u : local < sl_nb[a] ? sl_r0[a] + local : sp.ins_cl_ids[sl_i0[a] + (local - sl_nb[a])];
-        uint2 g1[1][NG];
-        float o1[1], t1[1];
-        uint32_t f1[1] = {0u};
-#pragma unroll
-        for (int q2 = 0; q2 < NG; ++q2)
-            g1[0][q2] = __ldg(reinterpret_cast<const uint2*>(sp.codes_il + il_granule_offset(m1[0], q2, NSQ)));
-        o1[0] = __ldg(reinterpret_cast<const float*>(sp.codes_il + il_offset_offset(m1[0], NSQ)));
-        const uint32_t fi = __ldg(reinterpret_cast<const uint16_t*>(sp.codes_il + il_fine_offset(m1[0], NSQ)));
-        float cterm[1] = {0.0f};
-        if (ok) {
-            const uint32_t c = sp.ctag[(uint64_t)qi * sp.P + a];
-            const float cd = sp.cdist[(uint64_t)qi * sp.P + a];
-            cterm[0] = 2.0f * __fadd_rn(__fadd_rn(cd, __ldg(sp.stationary + (uint64_t)c * F + fi)), __ldg(fdk + fi));
-        }
-        il_score<NSQ, HALF, 1, true>(tab, cterm, g1, o1, f1, m1, inv_scale, t1);
-        set_range(t1[0], ok);
-    }
-    for (uint32_t l = 0; l < L; ++l) {
-        __syncthreads();  // the previous cluster's cell terms are no longer read
-        if (tid == 0) {
-            const uint32_t c = sp.ctag[(uint64_t)qi * sp.P + l];
-            s_c = c;
-            s_cdl = sp.cdist[(uint64_t)qi * sp.P + l];
-            s_r0 = s_r1 = s_i0 = s_i1 = 0;
-            if (c < sp.C) {
-                s_r0 = sp.cell_start[(uint64_t)c * F];
-                s_r1 = sp.cell_start[(uint64_t)c * F + F];
-                if (sp.ins_cl_start) {
-                    s_i0 = sp.ins_cl_start[c];
-                    s_i1 = sp.ins_cl_start[c + 1];
+            for (int j = 0; j < R; ++j) {
+                const uint32_t ps = min((uint32_t)((float)((i0 + j * NT) & ~3u) * step), N - 1);
+                uint32_t a = 0, b = L;  // the slot holding position ps
+                while (b - a > 1) {
+                    const uint32_t mid = (a + b) >> 1;
+                    if (sl_start[mid] <= ps) a = mid;
+                    else b = mid;
                 }
-            }
-        }
-        __syncthreads();
-        const uint32_t c = s_c;
-        if (c >= sp.C) break;  // the probed clusters fill a prefix of the slots
-        const uint32_t r0 = s_r0, r1 = s_r1, i0 = s_i0, ni = s_i1 - s_i0, nrec = r1 - r0;
-        if (nrec + ni == 0) continue;
-        // srow[f] = 2 * cell_dist of cell f, cell_dist = (cd + stationary) + fd
-        // (puck_index.cpp:539-540)
-        const float cdl = s_cdl;
-        if ((F & 3u) == 0) {
-            const float4* st4 = reinterpret_cast<const float4*>(sp.stationary + (uint64_t)c * F);
-            const float4* fd4 = reinterpret_cast<const float4*>(fdk);
-            float4* s4 = reinterpret_cast<float4*>(srow);
-            for (uint32_t i = tid; i < (F >> 2); i += kSplitThreads) {
-                const float4 a = __ldg(st4 + i), b = __ldg(fd4 + i);
-                s4[i] = make_float4(2.0f * __fadd_rn(__fadd_rn(cdl, a.x), b.x),
-                                    2.0f * __fadd_rn(__fadd_rn(cdl, a.y), b.y),
-                                    2.0f * __fadd_rn(__fadd_rn(cdl, a.z), b.z),
-                                    2.0f * __fadd_rn(__fadd_rn(cdl, a.w), b.w));
-            }
-        } else {
-            for (uint32_t i = tid; i < F; i += kSplitThreads)
-                srow[i] = 2.0f * __fadd_rn(__fadd_rn(cdl, sp.stationary[(uint64_t)c * F + i]), fdk[i]);
-        }
-        __syncthreads();
-        if (nrec > 0) {
-            const uint32_t b0 = r0 >> 5, nblk = ((r1 - 1) >> 5) - b0 + 1;
-            const uint32_t steps = (nblk + NW * RB - 1) / (NW * RB);
-            // step j: warp w takes record blocks j * NW * RB + r * NW + w of the cluster
-            auto load = [&](uint32_t j, uint2 (&g)[RB][NG], float (&o)[RB], uint32_t (&f)[RB],
-                            uint32_t (&m)[RB], bool (&v)[RB]) {
-#pragma unroll
-                for (int r = 0; r < RB; ++r) {
-                    const uint32_t bi = j * (NW * RB) + r * NW + warp;
-                    m[r] = (b0 + bi) * 32u + lane;
-                    v[r] = bi < nblk && m[r] - r0 < nrec;
-                    if (bi < nblk) {
-                        const unsigned char* rec = sp.codes_il + (uint64_t)(b0 + bi) * kBlk;
-#pragma unroll
-                        for (int q2 = 0; q2 < NG; ++q2)
-                            g[r][q2] = __ldg(reinterpret_cast<const uint2*>(rec + q2 * 256 + 8 * lane));
-                        o[r] = __ldg(reinterpret_cast<const float*>(rec + 32 * kG + 4 * lane));
-                        f[r] = v[r] ? __ldg(reinterpret_cast<const uint16_t*>(rec + 32 * kG + 128 + 2 * lane))
-                                    : 0u;
-                    } else {
-#pragma unroll
-                        for (int q2 = 0; q2 < NG; ++q2) g[r][q2] = make_uint2(0u, 0u);
-                        o[r] = 0.0f;
-                        f[r] = 0u;
-                    }
-                }
-            };
-            // bulk L2 prefetch of step j's record blocks (one copy engine request by
-            // thread 0), kSplitAhead + 1 steps before their loads are issued
-            auto prefetch = [&](uint32_t j) {
-                if (kSplitAhead >= 0 && tid == 0 && j < steps) {
-                    const uint32_t first = j * (NW * RB);
-                    const uint32_t cnt = min((uint32_t)(NW * RB), nblk - first);
-                    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(
-                                     sp.codes_il + (uint64_t)(b0 + first) * kBlk),
-                                 "r"(cnt * kBlk)
-                                 : "memory");
-                }
-            };
-            for (int j = 1; j <= kSplitAhead; ++j) prefetch((uint32_t)j);
-            // two register sets, A and B, in turn: step j + 1's loads go into one set
-            // while step j is scored from the other (no copies between steps)
-            uint2 ga[RB][NG], gb[RB][NG];
-            float oa[RB], ob[RB];
-            uint32_t fa[RB], fb[RB], ma[RB], mb[RB];
-            bool va[RB], vb[RB];
-            auto emit = [&](const uint2 (&g)[RB][NG], const float (&o)[RB], const uint32_t (&f)[RB],
-                            const uint32_t (&m)[RB], const bool (&v)[RB]) {
-                float t[RB];
-                il_score<NSQ, HALF, RB, true>(tab, srow, g, o, f, m, inv_scale, t);
-#pragma unroll
-                for (int r = 0; r < RB; ++r)
-                    if (v[r]) {
-                        out[pos + (m[r] - r0)] = t[r];
-                        atomicAdd(&hist[split_bin(t[r], lo, scale)], 1u);
-                    }
-            };
-            load(0, ga, oa, fa, ma, va);
-            for (uint32_t j = 0; j < steps; j += 2) {
-                prefetch(j + kSplitAhead + 1);
-                if (j + 1 < steps) load(j + 1, gb, ob, fb, mb, vb);
-                emit(ga, oa, fa, ma, va);
-                if (j + 1 < steps) {
-                    prefetch(j + kSplitAhead + 2);
-                    if (j + 2 < steps) load(j + 2, ga, oa, fa, ma, va);
-                    emit(gb, ob, fb, mb, vb);
-                }
-            }
-            pos += nrec;
-        }
-        // realtime: the cluster's inserted records (gathered from the interleaved copy)
-        for (uint32_t v0 = 0; v0 < ni; v0 += kSplitThreads * RB) {
-            uint2 g[RB][NG];
-            float o[RB], t[RB];
-            uint32_t f[RB], m[RB];
-            bool v[RB];
-#pragma unroll
-            for (int r = 0; r < RB; ++r) {
-                const uint32_t vi = v0 + r * kSplitThreads + tid;
-                v[r] = vi < ni;
-                m[r] = v[r] ? sp.ins_cl_ids[i0 + vi] : 0u;
+                const uint32_t local = ps - sl_start[a], nb = sl_nb[a], r0 = sl_r0[a];
+                if (local < nb)
+                    m[j] = min(max(((r0 + local) & ~31u) + lane, r0), r0 + nb - 1);
+                else
+                    m[j] = sp.ins_cl_ids[sl_i0[a] + (local - nb)];
+                const uint32_t fi =
+                    __ldg(reinterpret_cast<const uint16_t*>(sp.codes_il + il_fine_offset(m[j], NSQ)));
 #pragma unroll
                 for (int q2 = 0; q2 < NG; ++q2)
-                    g[r][q2] = __ldg(reinterpret_cast<const uint2*>(sp.codes_il + il_granule_offset(m[r], q2, NSQ)));
-                o[r] = __ldg(reinterpret_cast<const float*>(sp.codes_il + il_offset_offset(m[r], NSQ)));
-                f[r] = v[r] ? __ldg(reinterpret_cast<const uint16_t*>(sp.codes_il + il_fine_offset(m[r], NSQ)))
-                            : 0u;
+                    g[j][q2] = __ldg(
+                        reinterpret_cast<const uint2*>(sp.codes_il + il_granule_offset(m[j], q2, NSQ)));
+                o[j] = __ldg(reinterpret_cast<const float*>(sp.codes_il + il_offset_offset(m[j], NSQ)));
+                cterm[j] = a < sp.lay.group
+                               ? srow[a * Fp + fi]
+                               : 2.0f * __fadd_rn(__fadd_rn(sl_cd[a], __ldg(sp.stationary +
+                                                                            (uint64_t)sl_c[a] * F + fi)),
+                                                  __ldg(fdk + fi));
+                f[j] = j;
             }
-            il_score<NSQ, HALF, RB, true>(tab, srow, g, o, f, m, inv_scale, t);
+            il_score<NSQ, HALF, R, true>(tab, cterm, g, o, f, m, inv_scale, t);
 #pragma unroll
-            for (int r = 0; r < RB; ++r)
-                if (v[r]) {
-                    out[pos + v0 + r * kSplitThreads + tid] = t[r];
-                    atomicAdd(&hist[split_bin(t[r], lo, scale)], 1u);
+            for (int j = 0; j < R; ++j) keys[i0 + j * NT] = filter_key(t[j], i0 + j * NT);
+        };
+        uint32_t i0 = tid;
+        for (; i0 + 4 * NT <= S + tid; i0 += 4 * NT) sample(i0, std::integral_constant<int, 4>());
+        if (i0 < S) sample(i0, std::integral_constant<int, 2>());
+        __syncthreads();
+        const uint64_t cut = block_cut_bound<NT>(keys, S, min(sample_rank(S, T, N), S),
+                                                 reinterpret_cast<uint32_t*>(keys + S), k_red);
+        if (cut != kKeyMax) tau = key_value(cut);
+    }
+    const uint32_t lanes_below = (1u << lane) - 1;
+    // keeps the records v with t at or below the bound, as (t bits, id): the warp's take
+    // consecutive slots
+    auto append = [&](const auto& t, const auto& m, const auto& v) {
+        constexpr int R = (int)(sizeof(t) / sizeof(t[0]));
+        unsigned b[R];
+        uint32_t nk = 0;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            b[r] = __ballot_sync(0xffffffffu, v[r] && t[r] <= tau);
+            nk += __popc(b[r]);
+        }
+        if (nk == 0) return;
+        uint32_t at = 0;
+        if (lane == 0) at = atomicAdd(&k_count, nk);
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (at + nk > cap) return;  // the buffer is full: the query will be left
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            if (b[r] >> lane & 1u)
+                keys[at + __popc(b[r] & lanes_below)] = ((uint64_t)__float_as_uint(t[r]) << 32) | m[r];
+            at += __popc(b[r]);
+        }
+    };
+    for (uint32_t g0 = 0; g0 < L; g0 += sp.lay.group) {
+        const uint32_t g1 = min(g0 + sp.lay.group, L);
+        __syncthreads();  // the previous group's cell terms (the sampled keys) are no longer read
+        if (g0 > 0) fill_rows(g0, g1);
+        __syncthreads();
+        // Cluster by cluster, without barriers: the warp takes record blocks w, w + NW, ...
+        // of RB blocks each, w rotating so that the clusters' last blocks spread over the
+        // warps. Two register sets, A and B, in turn: step j + 1's loads go into one set
+        // while step j is scored from the other (no copies between steps).
+        for (uint32_t l = g0; l < g1; ++l) {
+            const uint32_t nb = sl_nb[l], r0 = sl_r0[l];
+            if (nb == 0) continue;
+            const uint32_t nblk = (r0 + nb - 1) / 32 - r0 / 32 + 1;
+            const float* const row = srow + (l - g0) * Fp;
+            uint32_t bi = ((warp + l) % NW) * RB;
+            // a step's loads: whole steps, the blocks past the cluster's last are dropped
+            const unsigned char* rec = sp.codes_il + (uint64_t)(r0 / 32 + bi) * kBlk;
+            const unsigned char *pg = rec + 8 * lane, *po = rec + 32 * kG + 4 * lane,
+                                *pf = rec + 32 * kG + 128 + 2 * lane;
+            constexpr uint32_t kStep = NW * RB * kBlk;
+            auto load = [&](uint2 (&g)[RB][NG], float (&o)[RB], uint32_t (&f)[RB]) {
+#pragma unroll
+                for (int r = 0; r < RB; ++r) {
+#pragma unroll
+                    for (int q2 = 0; q2 < NG; ++q2)
+                        g[r][q2] = __ldg(reinterpret_cast<const uint2*>(pg + r * kBlk + q2 * 256));
+                    o[r] = __ldg(reinterpret_cast<const float*>(po + r * kBlk));
+                    f[r] = __ldg(reinterpret_cast<const uint16_t*>(pf + r * kBlk));
                 }
-        }
-        pos += ni;
-    }
-    __syncthreads();
-    // the cut: the first bin at which the running count reaches T (every bin when
-    // the query has no more than T records)
-    uint32_t bstar = kSplitBins - 1;
-    if (pos > T) {
-        constexpr int PB = kSplitBins / kSplitThreads;
-        uint32_t cb[PB], run = 0;
+                pg += kStep;
+                po += kStep;
+                pf += kStep;
+            };
+            uint32_t u = (r0 & ~31u) + bi * 32 + lane - r0;  // the lane's first record, from r0
+            auto emit = [&](const uint2 (&g)[RB][NG], const float (&o)[RB], const uint32_t (&f)[RB]) {
+                uint32_t m[RB], fc[RB], ln[RB];
+                bool v[RB];
+                float t[RB];
 #pragma unroll
-        for (int j = 0; j < PB; ++j) {
-            cb[j] = hist[tid * PB + j];
-            run += cb[j];
-        }
-        uint32_t incl = run;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += y;
-        }
-        if (lane == 31) s_red[warp] = incl;
-        __syncthreads();
-        uint32_t below = incl - run;
-        for (int w = 0; w < warp; ++w) below += s_red[w];
-        if (below < T && T <= below + run) {
-#pragma unroll
-            for (int j = 0; j < PB; ++j) {
-                if (below < T && T <= below + cb[j]) s_bin = tid * PB + j;
-                below += cb[j];
+                for (int r = 0; r < RB; ++r) {
+                    m[r] = r0 + u + r * 32;
+                    v[r] = u + r * 32 < nb;
+                    fc[r] = min(f[r], F - 1);  // (a dropped record's may be anything)
+                    ln[r] = lane;
+                }
+                il_score<NSQ, HALF, RB, true>(tab, row, g, o, fc, ln, inv_scale, t);
+                append(t, m, v);
+                u += NW * RB * 32;
+            };
+            uint2 ga[RB][NG], gb[RB][NG];
+            float oa[RB], ob[RB];
+            uint32_t fa[RB], fb[RB];
+            if (bi < nblk) load(ga, oa, fa);
+            for (; bi < nblk; bi += 2 * NW * RB) {
+                if (bi + NW * RB < nblk) load(gb, ob, fb);
+                emit(ga, oa, fa);
+                if (bi + NW * RB < nblk) {
+                    if (bi + 2 * NW * RB < nblk) load(ga, oa, fa);
+                    emit(gb, ob, fb);
+                }
             }
         }
-        __syncthreads();
-        bstar = s_bin;
-    }
-    // ---- pick: the records at or below the cut bin, read back from this block's own
-    // distances (recently written, mostly still in L2), as (t bits, position) keys in
-    // the table's place; positions to memory ids; the exact T smallest (t, id) out.
-    __syncthreads();  // the table, the cell terms and the histogram are no longer read
-    constexpr uint32_t kKeys = split_max_keys(false);
-    uint64_t* keys = reinterpret_cast<uint64_t*>(tab);
-    uint32_t* khist = hist;  // [kHistBins] block_kth_hist scratch
-    // candidates: each thread marks its 16 values of a step, a warp scan of the marks
-    // gives each thread its first slot (one shared atomic per warp and step)
-    const float4* tb4 = reinterpret_cast<const float4*>(out);  // out is 16-byte aligned
-    const uint32_t n4 = (N + 3) / 4;
-    for (uint32_t i0 = 0; i0 < n4; i0 += kSplitThreads * 4) {
-        float4 x[4];
+        // realtime: the clusters' inserted records (gathered from the interleaved copy)
+        for (uint32_t l = g0; sp.ins_cl_start != nullptr && l < g1; ++l) {
+            const uint32_t i0 = sl_i0[l], ni = sl_start[l + 1] - sl_start[l] - sl_nb[l];
+            const float* const row = srow + (l - g0) * Fp;
+            for (uint32_t v0 = 0; v0 < ni; v0 += NT) {
+                const uint32_t vi = v0 + tid;
+                const bool v[1] = {vi < ni};
+                const uint32_t m1[1] = {v[0] ? sp.ins_cl_ids[i0 + vi] : 0u};
+                uint2 g[1][NG];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const uint32_t i = i0 + u * kSplitThreads + tid;
-            x[u] = i < n4 ? __ldcg(tb4 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-        uint32_t mask = 0;
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const uint32_t i = i0 + u * kSplitThreads + tid;
-            const float tv[4] = {x[u].x, x[u].y, x[u].z, x[u].w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const bool keep = i < n4 && i * 4 + e < N && split_bin(tv[e], lo, scale) <= bstar;
-                mask |= keep ? 1u << (u * 4 + e) : 0u;
+                for (int q2 = 0; q2 < NG; ++q2)
+                    g[0][q2] = __ldg(
+                        reinterpret_cast<const uint2*>(sp.codes_il + il_granule_offset(m1[0], q2, NSQ)));
+                const float o[1] = {
+                    __ldg(reinterpret_cast<const float*>(sp.codes_il + il_offset_offset(m1[0], NSQ)))};
+                const uint32_t f[1] = {v[0] ? __ldg(reinterpret_cast<const uint16_t*>(
+                                                  sp.codes_il + il_fine_offset(m1[0], NSQ)))
+                                            : 0u};
+                float t[1];
+                il_score<NSQ, HALF, 1, true>(tab, row, g, o, f, m1, inv_scale, t);
+                append(t, m1, v);
             }
-        }
-        const uint32_t c = __popc(mask);
-        uint32_t incl = c;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += y;
-        }
-        uint32_t base = 0;
-        if (lane == 31 && incl) base = atomicAdd(&k_count, incl);
-        base = __shfl_sync(0xffffffffu, base, 31);
-        uint32_t slot = base + incl - c;
-        while (mask) {
-            const int b = __ffs(mask) - 1;
-            mask &= mask - 1;
-            const int u = b >> 2, e = b & 3;
-            const uint32_t ps = (i0 + u * kSplitThreads + tid) * 4 + e;
-            float tv = 0.0f;  // x[u] element e, by selects (no local-memory array)
-#pragma unroll
-            for (int uu = 0; uu < 4; ++uu)
-                if (uu == u) tv = e == 0 ? x[uu].x : e == 1 ? x[uu].y : e == 2 ? x[uu].z : x[uu].w;
-            if (slot < kKeys) keys[slot] = ((uint64_t)__float_as_uint(tv) << 32) | ps;
-            ++slot;
         }
     }
     __syncthreads();
     const uint32_t m = k_count;
-    if (m > kKeys) {  // too many records in the cut bin: k_scan_il takes the query
-        if (tid == 0) sp.qflag[qi] = 0;
+    if (m > cap || m < min(T, N)) {  // the bound was too high or too low
+        if (tid == 0) sp.todo[atomicAdd(sp.ntodo, 1u)] = qi;
         return;
     }
-    // positions to memory ids: the slot holding the position (binary search), then the
-    // base record or the inserted one
-    for (uint32_t i = tid; i < m; i += kSplitThreads) {
-        const uint64_t k = keys[i];
-        const uint32_t ps = (uint32_t)k;
-        const uint32_t a = slot_of(ps);
-        const uint32_t local = ps - sl_start[a];
-        const uint32_t id =
-            local < sl_nb[a] ? sl_r0[a] + local : sp.ins_cl_ids[sl_i0[a] + (local - sl_nb[a])];
-        keys[i] = filter_key(__uint_as_float((uint32_t)(k >> 32)), id);
-    }
-    __syncthreads();
-    // the exact T smallest: the keys up to the T-th (all of them when m <= T), written
-    // unordered like k_scan_il's
-    const uint64_t bound =
-        m > T ? block_kth_hist<kSplitThreads>(keys, m, T, khist, k_red, &k_cnt, k_hist256, k_sel) + 1
-              : kKeyMax;
-    for (uint32_t i0 = 0; i0 < m; i0 += kSplitThreads) {
-        const uint32_t i = i0 + tid;
-        const uint64_t k = i < m ? keys[i] : kKeyMax;
-        const bool keep = k < bound;
-        const unsigned b = __ballot_sync(0xffffffffu, keep);
-        if (b) {
-            uint32_t base = 0;
-            if (lane == __ffs(b) - 1) base = atomicAdd(&k_out, (uint32_t)__popc(b));
-            base = __shfl_sync(0xffffffffu, base, __ffs(b) - 1);
-            if (keep) {
-                const uint32_t slot = base + __popc(b & ((1u << lane) - 1));
-                sp.hdist[(uint64_t)qi * T + slot] = key_value(k);
-                sp.htag[(uint64_t)qi * T + slot] = (uint32_t)k;
-            }
+    // the exact T smallest, written unordered like k_scan_il's; the table's place is free
+    auto put = [&](uint32_t slot, uint64_t k) {
+        sp.hdist[(uint64_t)qi * T + slot] = key_value(k);
+        sp.htag[(uint64_t)qi * T + slot] = (uint32_t)k;
+    };
+    // keys[i] below the bound go out, a ballot at a time; one atomic per warp
+    constexpr int kPer = 16;  // keys per thread in registers
+    uint32_t* hist = reinterpret_cast<uint32_t*>(tab);               // [kHistBins]
+    uint64_t* ties = reinterpret_cast<uint64_t*>(hist + kHistBins);  // keys of the T-th's bin
+    constexpr uint32_t kTies = 1024;
+    uint64_t k[kPer];
+    uint32_t lo = 0xFFFFFFFFu, hi = 0, bin = 0xFFFFFFFFu, shift = 0, below = m;
+    const bool regs = m <= (uint32_t)(kPer * NT);
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+        const uint32_t i = j * NT + tid;
+        const uint64_t x = regs && i < m ? keys[i] : 0ull;
+        k[j] = filter_key(__uint_as_float((uint32_t)(x >> 32)), (uint32_t)x);
+        if (regs && i < m) {
+            lo = min(lo, (uint32_t)(k[j] >> 32));
+            hi = max(hi, (uint32_t)(k[j] >> 32));
+        } else {
+            k[j] = kKeyMax;
         }
     }
-    __syncthreads();
-    const uint32_t outn = k_out;  // min(m, T)
-    for (uint32_t i = outn + tid; i < T; i += kSplitThreads) {
+    if (regs && m > T) {
+        // the bin of the T-th smallest among kHistBins between the smallest and the largest
+        lo = __reduce_min_sync(0xffffffffu, lo);
+        hi = __reduce_max_sync(0xffffffffu, hi);
+        if (lane == 0) {
+            k_red[warp] = lo;
+            k_red[NW + warp] = hi;
+        }
+        for (uint32_t b = tid; b < kHistBins; b += NT) hist[b] = 0;
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < NW; ++w) {
+            lo = min(lo, k_red[w]);
+            hi = max(hi, k_red[NW + w]);
+        }
+        shift = 32 - min(__clz(hi - lo), 32);
+        shift = shift > 10 ? shift - 10 : 0;
+        static_assert(kHistBins == 1024, "10 bits of the range");
+#pragma unroll
+        for (int j = 0; j < kPer; ++j)
+            if (j * NT + tid < m) atomicAdd(&hist[((uint32_t)(k[j] >> 32) - lo) >> shift], 1u);
+        __syncthreads();
+        constexpr uint32_t per = kHistBins / NT;
+        uint32_t c[per], sum = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < per; ++j) {
+            c[j] = hist[tid * per + j];
+            sum += c[j];
+        }
+        uint32_t inc = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += y;
+        }
+        if (lane == 31) s_red[warp] = inc;
+        __syncthreads();
+        uint32_t bl = inc - sum;
+        for (int w = 0; w < warp; ++w) bl += s_red[w];
+        if (bl < T && T <= bl + sum) {
+#pragma unroll
+            for (uint32_t j = 0; j < per; ++j) {
+                if (bl < T && T <= bl + c[j]) {
+                    k_red[0] = tid * per + j;
+                    k_red[1] = bl;
+                    k_red[2] = c[j];
+                }
+                bl += c[j];
+            }
+        }
+        __syncthreads();
+        bin = k_red[0];
+        below = k_red[1];
+    }
+    if (regs && (m <= T || k_red[2] <= kTies)) {
+        // below the bin: out; the bin's own: the first by rank fill up to T
+        const uint32_t lim = min(m, T) - (m > T ? below : m);
+        uint32_t nout = 0;
+        unsigned in[kPer];
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            const bool have = j * NT + tid < m;
+            const uint32_t mybin = m > T ? ((uint32_t)(k[j] >> 32) - lo) >> shift : 0u;
+            in[j] = __ballot_sync(0xffffffffu, have && mybin < bin);
+            nout += __popc(in[j]);
+            if (have && mybin == bin) ties[atomicAdd(&k_cnt, 1u)] = k[j];
+        }
+        uint32_t at = 0;
+        if (lane == 0) at = atomicAdd(&k_out, nout);
+        at = __shfl_sync(0xffffffffu, at, 0);
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            if (in[j] >> lane & 1u) put(at + __popc(in[j] & ((1u << lane) - 1)), k[j]);
+            at += __popc(in[j]);
+        }
+        if (lim > 0) {
+            __syncthreads();
+            const uint32_t nt = k_cnt;
+            for (uint32_t i = tid; i < nt; i += NT) {
+                const uint64_t x = ties[i];
+                uint32_t rank = 0;
+                for (uint32_t u = 0; u < nt; ++u) rank += ties[u] < x ? 1u : 0u;
+                if (rank < lim) put(below + rank, x);
+            }
+        }
+    } else {
+        // more keys than the registers take, or in the T-th's bin
+        __syncthreads();
+        for (uint32_t i = tid; i < m; i += NT) {
+            const uint64_t x = keys[i];
+            keys[i] = filter_key(__uint_as_float((uint32_t)(x >> 32)), (uint32_t)x);
+        }
+        __syncthreads();
+        const uint64_t bound =
+            m > T ? block_kth_hist<NT>(keys, m, T, hist, k_red, &k_cnt, k_hist256, k_sel) + 1 : kKeyMax;
+        for (uint32_t i0 = 0; i0 < m; i0 += NT) {
+            const uint32_t i = i0 + tid;
+            const uint64_t x = i < m ? keys[i] : kKeyMax;
+            const unsigned b = __ballot_sync(0xffffffffu, x < bound);
+            uint32_t at = 0;
+            if (lane == 0 && b) at = atomicAdd(&k_out, (uint32_t)__popc(b));
+            at = __shfl_sync(0xffffffffu, at, 0);
+            if (x < bound) put(at + __popc(b & ((1u << lane) - 1)), x);
+        }
+    }
+    const uint32_t outn = min(m, T);
+    for (uint32_t i = outn + tid; i < T; i += NT) {
         sp.hdist[(uint64_t)qi * T + i] = sentinel_f();
         sp.htag[(uint64_t)qi * T + i] = kNoLabel;
     }
@@ -1915,70 +1927,27 @@ size_t scan_smem_bytes_half(const DeviceIndex& ix, uint32_t T) {
 uint32_t scan_max_filter_topk() { return kMaxCap - kRound - 1024; }
 
 cudaError_t launch_scan_order(const DeviceIndex& ix, uint32_t n, Scratch& s, cudaStream_t stream) {
-    if (s.order == nullptr || s.wbucket == nullptr) return cudaErrorInvalidValue;
+    if (s.order == nullptr || s.wbin == nullptr) return cudaErrorInvalidValue;
     k_scan_work<<<(n + 255) / 256, 256, 0, stream>>>(s.ctag, s.status, ix.cell_start,
                                                      ix.ins_n ? ix.ins_cl_start : nullptr, n, s.P,
-                                                     ix.C, ix.F, s.wbucket);
-    k_scan_order<<<1, kOrderThreads, 0, stream>>>(s.wbucket, n, s.order);
+                                                     ix.C, ix.F, s.wbin);
+    k_scan_order<<<1, kOrderThreads, 0, stream>>>(s.wbin, n, s.order, s.ntodo);
     return cudaGetLastError();
 }
 
-// Shared memory of k_scan_score: the table, the query, then the compact table being
-// built or the cell terms and the histogram.
-static size_t split_score_smem(const DeviceIndex& ix, bool half) {
-    (void)half;  // the FP16 table takes the FP32 table's slots
-    const size_t stage = sizeof(float) * ix.nsq * 257;
-    const size_t work = il_srow_bytes(ix.F) + sizeof(uint32_t) * (kSplitBins + 4 * kSplitMaxSlots + 1);
-    return il_table_bytes(false) + il_query_bytes(ix.d) + (stage > work ? stage : work);
-}
-
-bool scan_split_possible(const DeviceIndex& ix, uint32_t T) {
-    return il_applies(ix.nsq) && split_score_smem(ix, false) <= 220 * 1024 &&
-           T < split_max_keys(false);
+static SplitLayout split_choice(const DeviceIndex& ix, uint32_t P, uint32_t T) {
+    const SplitLayout two = split_layout(ix.nsq, ix.d, ix.F, P, kSplitBudget2);
+    if (two.bytes && two.cap >= split_need(T)) return two;
+    const SplitLayout one = split_layout(ix.nsq, ix.d, ix.F, P, kSplitBudget1);
+    return one.bytes && one.cap >= T + 2 * kSplitThreads + 1024 ? one : SplitLayout{};
 }
 
 bool scan_split_applies(const DeviceIndex& ix, const Scratch& s) {
-    return ix.codes_il != nullptr && s.tbuf != nullptr && s.tcap > 0 && scan_split_possible(ix, s.T);
-}
-
-static SplitParams split_params(const DeviceIndex& ix, uint32_t n, Scratch& s) {
-    SplitParams sp;
-    sp.ctag = s.ctag;
-    sp.cdist = s.cdist;
-    sp.status = s.status;
-    sp.cell_start = ix.cell_start;
-    sp.ins_cl_start = ix.ins_n ? ix.ins_cl_start : nullptr;
-    sp.ins_cl_ids = ix.ins_cl_ids;
-    sp.stationary = ix.stationary;
-    sp.fd_by_fine = s.dots;
-    sp.q = s.q;
-    sp.qnorm = s.qnorm;
-    sp.codebook = ix.codebook;
-    sp.codes_il = ix.codes_il;
-    sp.order = s.order;
-    sp.qcnt = s.qcnt;
-    sp.qoff = s.qoff;
-    sp.qflag = s.qflag;
-    sp.cut = s.cut;
-    sp.tbuf = s.tbuf;
-    sp.hdist = s.hdist;
-    sp.htag = s.htag;
-    sp.hcnt = s.hcnt;
-    sp.counters = s.counters;
-    sp.tcap = s.tcap;
-    sp.n = n;
-    sp.d = ix.d;
-    sp.C = ix.C;
-    sp.F = ix.F;
-    sp.lsq = ix.lsq;
-    sp.P = s.P;
-    sp.T = s.T;
-    sp.codebook_max = ix.codebook_max;
-    return sp;
+    return il_applies(ix.nsq) && ix.codes_il != nullptr && split_choice(ix, s.P, s.T).bytes != 0;
 }
 
 static cudaError_t launch_fused(const DeviceIndex& ix, uint32_t n, Scratch& s, bool half_lut,
-                                const uint32_t* done, cudaStream_t stream) {
+                                bool left, cudaStream_t stream) {
     ScanParams p;
     p.q = s.q;
     p.qnorm = s.qnorm;
@@ -2012,12 +1981,17 @@ static cudaError_t launch_fused(const DeviceIndex& ix, uint32_t n, Scratch& s, b
     p.err = s.tc_err;
     p.ins_cl_start = ix.ins_n ? ix.ins_cl_start : nullptr;
     p.ins_cl_ids = ix.ins_cl_ids;
-    p.done = done;
+    p.todo = left ? s.todo : nullptr;
+    p.ntodo = s.ntodo;
+    p.n = n;
     const size_t smem = half_lut ? scan_smem_bytes_half(ix, s.T) : scan_smem_bytes(ix, s.T);
     const uint32_t nw = ix.code_stride / 4;
+    // the queries the split scan left are few, as a rule none: a grid of the blocks that
+    // fit the chip loops over them
+    const uint32_t fits = 2u * (uint32_t)sm_count();
     auto launch = [&](void (*kernel)(ScanParams), int threads) {
         ensure_max_dynamic_smem(kernel, 220 * 1024);
-        kernel<<<n, threads, smem, stream>>>(p);
+        kernel<<<left && n > fits ? fits : n, threads, smem, stream>>>(p);
     };
     if (il_applies(ix.nsq)) {
         if (ix.codes_il == nullptr) return cudaErrorInvalidValue;
@@ -2049,24 +2023,41 @@ static cudaError_t launch_fused(const DeviceIndex& ix, uint32_t n, Scratch& s, b
     return cudaGetLastError();
 }
 
-cudaError_t launch_scan_prepare(const DeviceIndex& ix, uint32_t n, Scratch& s, bool half_lut,
-                                cudaStream_t stream) {
-    if (!scan_split_applies(ix, s)) return cudaSuccess;
-    (void)half_lut;
-    const SplitParams sp = split_params(ix, n, s);
-    k_split_counts<<<(n + 255) / 256, 256, 0, stream>>>(sp);
-    k_split_offsets<<<1, 1024, 0, stream>>>(sp);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_scan_records(const DeviceIndex& ix, uint32_t n, Scratch& s, bool half_lut,
                                 cudaStream_t stream) {
-    if (!scan_split_applies(ix, s)) return launch_fused(ix, n, s, half_lut, nullptr, stream);
-    const SplitParams sp = split_params(ix, n, s);
-    const size_t smem = split_score_smem(ix, half_lut);
+    if (!scan_split_applies(ix, s)) return launch_fused(ix, n, s, half_lut, false, stream);
+    SplitParams sp;
+    sp.ctag = s.ctag;
+    sp.cdist = s.cdist;
+    sp.status = s.status;
+    sp.cell_start = ix.cell_start;
+    sp.ins_cl_start = ix.ins_n ? ix.ins_cl_start : nullptr;
+    sp.ins_cl_ids = ix.ins_cl_ids;
+    sp.stationary = ix.stationary;
+    sp.fd_by_fine = s.dots;
+    sp.q = s.q;
+    sp.qnorm = s.qnorm;
+    sp.codebook = ix.codebook;
+    sp.codes_il = ix.codes_il;
+    sp.order = s.order;
+    sp.todo = s.todo;
+    sp.ntodo = s.ntodo;
+    sp.hdist = s.hdist;
+    sp.htag = s.htag;
+    sp.hcnt = s.hcnt;
+    sp.counters = s.counters;
+    sp.n = n;
+    sp.d = ix.d;
+    sp.C = ix.C;
+    sp.F = ix.F;
+    sp.lsq = ix.lsq;
+    sp.P = s.P;
+    sp.T = s.T;
+    sp.codebook_max = ix.codebook_max;
+    sp.lay = split_choice(ix, s.P, s.T);
     auto score = [&](void (*kernel)(SplitParams)) {
         ensure_max_dynamic_smem(reinterpret_cast<const void*>(kernel), 220 * 1024);
-        kernel<<<n, kSplitThreads, smem, stream>>>(sp);
+        kernel<<<n, kSplitThreads, sp.lay.bytes, stream>>>(sp);
     };
     switch (ix.nsq) {
 #define PGPU_SPLIT(N)                           \
@@ -2085,9 +2076,7 @@ cudaError_t launch_scan_records(const DeviceIndex& ix, uint32_t n, Scratch& s, b
 cudaError_t launch_scan_finish(const DeviceIndex& ix, uint32_t n, Scratch& s, bool half_lut,
                                cudaStream_t stream) {
     if (!scan_split_applies(ix, s)) return cudaSuccess;
-    // the fused kernel takes the queries the split scan did not answer (its blocks for
-    // answered queries return at once)
-    return launch_fused(ix, n, s, half_lut, s.qflag, stream);
+    return launch_fused(ix, n, s, half_lut, true, stream);
 }
 
 }  // namespace pgpu

@@ -1,0 +1,64 @@
+"""Scan mode's filter stage against the oracle's restatement, bit for bit, where its
+paths change hands: every record kept or a sampled bound, buffers that overflow and
+queries with more clusters than slots (both answered by the fused kernel), filter_topk
+of 1, above the buffer of two blocks per SM, and above the records of the probed
+clusters; rows of cell terms that are not whole float4s; groups of clusters.
+"""
+import os
+import tempfile
+
+import numpy as np
+import pytest
+
+import oracle
+from puck_gb300 import index_io, native
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _lib():
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+    native.load(build_if_missing=True)
+
+
+def _index(tmp, n, d, C, F, nsq, seed, distinct):
+    import torch
+    from puck_gb300 import builder
+    base = builder.gmm(n, d, 64, "unit", seed)
+    if distinct:
+        base = base[torch.arange(n, device=base.device) % distinct].contiguous()
+    a = builder.build_index(base, C, F, nsq, False, train_sample=min(n, 65536), iters=4,
+                            pq_sample=min(n, 32768), seed=seed)
+    index_io.write_index(tmp, base=a["base"], coarse=a["coarse"], fine=a["fine"],
+                         cell_assign=a["cell_assign"], filter_codebook=a["filter_codebook"],
+                         filter_offsets=a["filter_offsets"], filter_codes=a["filter_codes"],
+                         whether_norm=False)
+    return builder.gmm(70, d, 64, "unit", seed, row_seed=seed + 7).cpu().numpy()
+
+
+@pytest.mark.parametrize("n,d,C,F,nsq,P,T,distinct", [
+    (30_000, 64, 12, 40, 16, 1, 100, 0),     # a few thousand records: all kept
+    (60_000, 64, 12, 37, 16, 12, 1, 0),      # sampled, one candidate, odd rows
+    (60_000, 64, 40, 33, 16, 40, 1500, 0),   # several groups of clusters
+    (200_000, 32, 6, 50, 8, 6, 300, 0),      # several sampling passes
+    (40_000, 64, 10, 4600, 16, 10, 2048, 0),  # one block per SM
+    (9_000, 16, 5, 20, 4, 2, 2048, 0),       # close to all of the records, fewer for some
+    (60_000, 32, 8, 16, 8, 8, 200, 150),     # 150 distinct vectors: ties fill the buffer
+    (20_000, 32, 600, 10, 8, 600, 50, 0),    # more clusters than slots
+    (40_000, 96, 16, 2000, 24, 16, 700, 0),  # two clusters to a group
+])
+def test_scan_matches_oracle(n, d, C, F, nsq, P, T, distinct):
+    k = min(10, T)
+    with tempfile.TemporaryDirectory() as tmp:
+        q = _index(tmp, n, d, C, F, nsq, 5, distinct)
+        ix = native.GpuIndex(tmp, search_coarse_count=P, filter_topk=T, topk=k, max_batch=64,
+                             mode=native.PGPU_MODE_SCAN)
+        dist, ids = ix.search(q, k)
+        od, oi, st = oracle.OracleIndex(tmp).search_batch(q, k, P, T, topk_max=k,
+                                                          nthreads=os.cpu_count(), scan=True)
+        assert (st == 0).all()
+        assert np.array_equal(dist.view(np.uint32), od.view(np.uint32))
+        assert np.array_equal(ids, oi)

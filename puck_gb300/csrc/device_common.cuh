@@ -66,6 +66,79 @@ __device__ __forceinline__ void heap_reorder(float* hv, uint32_t* ht, uint32_t s
     }
 }
 
+// One lane's place in the subtree a heap round reads: lane i >= 1 owns node i (depth
+// floor(log2 i)) and lies on the way down when every strict ancestor (bits `above`) moves its
+// child up and those in `rights` move the right one.
+struct HeapLane {
+    int depth;
+    uint32_t off;
+    unsigned above, rights;
+};
+__device__ __forceinline__ HeapLane heap_lane() {
+    const uint32_t lane = threadIdx.x & 31;
+    HeapLane h;
+    h.depth = 31 - __clz(lane | 1);
+    h.off = lane - (1u << h.depth);  // lane 0 owns no node
+    h.above = h.rights = 0;
+    for (uint32_t i = lane; i > 1; i >>= 1) {
+        h.above |= 1u << (i >> 1);
+        if (i & 1) h.rights |= 1u << (i >> 1);
+    }
+    return h;
+}
+
+// MaxHeap insert of (v, tag) at slot f of heap[1..size] by one warp: heap_insert's steps
+// (the larger child moves up, the right one on equal values, until it is below v), five
+// levels per round. heap[i] = (value bits, tag): one 16-byte load holds both children of a
+// node. Returns the value that lands in slot f.
+__device__ __forceinline__ float warp_heap_insert(uint2* heap, uint32_t size, uint32_t f, float v,
+                                                  uint32_t tag, const HeapLane& hl) {
+    const int lane = threadIdx.x & 31;
+    float landed = v;
+    bool first = true;
+    while (2 * f <= size) {
+        const uint32_t node = (f << hl.depth) + hl.off;
+        const bool has = lane > 0 && 2 * node <= size;
+        const uint4 ch = reinterpret_cast<const uint4*>(heap)[has ? node : 0u];
+        const float lv = __uint_as_float(ch.x), rv = __uint_as_float(ch.z);
+        const bool right = has && 2 * node + 1 <= size && !(lv > rv);
+        const float cv = right ? rv : lv;
+        const bool stop = !has || cv < v;
+        const unsigned stops = __ballot_sync(0xffffffffu, stop);
+        const unsigned rights = __ballot_sync(0xffffffffu, right);
+        const bool on = lane > 0 && (rights & hl.above) == hl.rights && (stops & hl.above) == 0;
+        // the way goes on below this subtree from one lane at most
+        const uint32_t down = on && !stop && hl.depth == 4 ? 2 * node + (right ? 1u : 0u) : 0u;
+        f = __reduce_max_sync(0xffffffffu, down);
+        if (first) {
+            const float up = __shfl_sync(0xffffffffu, cv, 1);
+            landed = (stops & 2u) ? v : up;
+            first = false;
+        }
+        if (on)
+            heap[node] = stop ? make_uint2(__float_as_uint(v), tag)
+                              : make_uint2(__float_as_uint(cv), right ? ch.w : ch.y);
+        if (f == 0) {
+            __syncwarp();
+            return landed;
+        }
+    }
+    if (lane == 0) heap[f] = make_uint2(__float_as_uint(v), tag);
+    __syncwarp();
+    return landed;
+}
+
+// heap_reorder of heap[1..size] by one warp.
+__device__ inline void warp_heap_reorder(uint2* heap, uint32_t size, const HeapLane& hl) {
+    for (uint32_t hs = size; hs > 0; --hs) {
+        const uint2 top = heap[1], last = heap[hs];
+        __syncwarp();
+        warp_heap_insert(heap, hs - 1, 1, __uint_as_float(last.x), last.y, hl);
+        if ((threadIdx.x & 31) == 0) heap[hs] = top;
+        __syncwarp();
+    }
+}
+
 // ------------------------------------------------------------- block scans
 // Inclusive scan over a block of NW warps; `warp_tot` needs NW slots.
 template <int NW>

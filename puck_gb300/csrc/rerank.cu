@@ -13,7 +13,7 @@
 //
 // Selection: when no two of the topk+1 smallest distances are equal the heap's
 // output is just the ascending order, found by a bitonic sort of
-// (distance, position); otherwise thread 0 replays the heap exactly.
+// (distance, position); otherwise a warp replays the heap exactly.
 //
 // k_rerank_screen (precision form): the same result from fewer bytes. Each
 // candidate is first measured on a BF16 copy of its vector; with |x~ - x| <=
@@ -43,7 +43,7 @@ namespace {
 #define PGPU_RERANK_SCREEN_MIN_BLOCKS 8
 #endif
 constexpr int kThreads = PGPU_RERANK_THREADS;
-constexpr int kWarps = kThreads / 32;
+constexpr int kPqThreads = 512;  // the PQ table leaves two blocks per SM
 constexpr int kScreenThreads = PGPU_RERANK_SCREEN_THREADS;
 constexpr int kScreenWarps = kScreenThreads / 32;
 constexpr int kRows = 8;  // candidate rows per warp in flight (rows8_l2_exact)
@@ -68,6 +68,8 @@ struct RerankParams {
     const float* pq_offsets;
     const uint8_t* pq_codes;
     uint32_t pq_nsq, pq_lsq, pq_code_stride;
+    uint32_t work_bytes;  // shared memory before the query: sort arrays, before them the PQ table
+    int pq_table;         // the PQ table is in shared memory
     // a realtime index (RealtimeInsertPuckIndex) sums the PQ table subspace by
     // subspace in order (realtime_insert_puck_index.cpp:466-499), not in
     // lookup_dist_table's four partials
@@ -226,20 +228,64 @@ __device__ __forceinline__ void rows8_l2_exact(const float* const* rows, const f
         warp_l2_exact<8>(rows, q, d, lane, out);
 }
 
+// The exact MaxHeap(topk) fed with cnt distances in the given order (null: as they are), then
+// reorder(), written out; by one warp. heap: topk + 2 entries, 16-byte aligned. A ballot
+// finds the next distance below the top, so the steps are the insertions (about
+// topk (1 + ln(cnt / topk)) of them) and not the candidates; one thread doing all, with each
+// tag fetched from memory, took 0.2 ms for 1100 candidates and topk 100 (a query in that
+// path ended a whole batch's launch).
+__device__ __noinline__ void heap_replay(uint2* heap, const float* dist, const uint32_t* order,
+                                         uint32_t cnt, uint32_t topk, const uint32_t* tags,
+                                         const uint32_t* mem2local, float* od, uint32_t* oi) {
+    const uint32_t lane = threadIdx.x & 31;
+    const HeapLane hl = heap_lane();
+    for (uint32_t i = lane; i < topk + 2; i += 32) heap[i] = make_uint2(__float_as_uint(sentinel_f()), 0u);
+    __syncwarp();
+    float top = sentinel_f();
+    uint32_t dpc = topk;
+    for (uint32_t r0 = 0; r0 < cnt; r0 += 32) {
+        const uint32_t r = r0 + lane;
+        const uint32_t j = r < cnt ? (order ? order[r] : r) : 0u;
+        const float v = r < cnt ? dist[j] : sentinel_f();
+        unsigned todo = __ballot_sync(0xffffffffu, r < cnt && v < top);
+        while (todo) {
+            const int src = __ffs(todo) - 1;
+            warp_heap_insert(heap, topk, dpc > 0 ? dpc-- : 1u, __shfl_sync(0xffffffffu, v, src),
+                             __shfl_sync(0xffffffffu, j, src), hl);
+            top = __uint_as_float(heap[1].x);
+            // later candidates, still below the top
+            todo = __ballot_sync(0xffffffffu, (todo >> lane & 1u) && (int)lane > src && v < top);
+        }
+    }
+    warp_heap_reorder(heap, topk, hl);
+    const uint32_t rn = topk - dpc;
+    for (uint32_t i = lane; i < topk; i += 32) {
+        od[i] = __uint_as_float(heap[i + 1].x);
+        oi[i] = i < rn ? mem2local[tags[heap[i + 1].y]] : kNoLabel;
+    }
+}
+
 // PQ: the second-level PQ branch of rank_topN_points (puck_index.cpp:402-427): per
 // candidate (filter distance - |q|^2) + pq offset, then + lookup_dist_table over
 // the PQ table (get_dist_table, quantization.cpp:260-270), in the reference's
-// float order; the same heap semantics as the Puck-Flat branch.
+// float order; the same heap semantics as the Puck-Flat branch. Bound by the lookups: the
+// table in shared memory (random banks, about 3.4 wavefronts per warp-wide lookup) and code
+// rows by 16-byte loads; one-dimensional entries formed from the codebook at each lookup, and
+// the rows read a word at a time, took 0.62 ms for 1537 queries of 1100 candidates and 96 entries
+// each, with the heap by one thread; this form takes 0.23.
 template <bool PQ>
-__global__ __launch_bounds__(kThreads) void k_rerank(RerankParams p) {
+__global__ __launch_bounds__(PQ ? kPqThreads : kThreads) void k_rerank(RerankParams p) {
+    constexpr int NT = PQ ? kPqThreads : kThreads;
     extern __shared__ __align__(16) unsigned char smem[];
+    // the sort arrays take the table's place once the distances are there
     unsigned long long* okey = reinterpret_cast<unsigned long long*>(smem);  // [Tp]
-    float* qv = reinterpret_cast<float*>(okey + p.Tp);
-    float* dist = qv + p.d;                                   // [T]
-    float* sv = dist + p.T;                                   // [Tp]
-    uint32_t* si = reinterpret_cast<uint32_t*>(sv + p.Tp);    // [Tp]
-    uint32_t* opos = si + p.Tp;                               // [Tp]
-    float* pq_lut = reinterpret_cast<float*>(opos + p.Tp);    // [pq_nsq * 256] (PQ)
+    float* sv = reinterpret_cast<float*>(okey + p.Tp);                       // [Tp]
+    uint32_t* si = reinterpret_cast<uint32_t*>(sv + p.Tp);                   // [Tp]
+    uint32_t* opos = si + p.Tp;                                              // [Tp]
+    float* pq_lut = reinterpret_cast<float*>(smem);                          // [pq_nsq * 256] (PQ)
+    float* qv = reinterpret_cast<float*>(smem + p.work_bytes);
+    float* dist = qv + p.d;                                                  // [T]
+    uint32_t* stag = reinterpret_cast<uint32_t*>(dist + p.T);                // [T]
     __shared__ uint32_t sel_hist[256];
     __shared__ uint32_t sel_state[2];
     __shared__ uint32_t sel_count;
@@ -250,7 +296,7 @@ __global__ __launch_bounds__(kThreads) void k_rerank(RerankParams p) {
     const int32_t stq = p.status[qi];
     if (p.out_status && tid == 0) p.out_status[qi] = stq;
     if (stq != 0) {
-        for (uint32_t i = tid; i < topk; i += kThreads) {
+        for (uint32_t i = tid; i < topk; i += NT) {
             od[i] = sentinel_f();
             oi[i] = kNoLabel;
         }
@@ -258,27 +304,84 @@ __global__ __launch_bounds__(kThreads) void k_rerank(RerankParams p) {
     }
     const uint32_t cnt = p.hcnt[qi];
     const uint32_t* tags = p.htag + (uint64_t)qi * p.T;
-    for (uint32_t i = tid; i < p.d; i += kThreads) qv[i] = p.q[(uint64_t)qi * p.d + i];
-    {
-        // the candidates' memory ids in shared memory (one coalesced load)
-        uint32_t* stag = reinterpret_cast<uint32_t*>(pq_lut + (p.pq_lsq > 1 ? p.pq_nsq * 256 : 0));
-        for (uint32_t i = tid; i < cnt; i += kThreads) stag[i] = tags[i];
-        tags = stag;
+    for (uint32_t i = tid; i < p.d; i += NT) qv[i] = p.q[(uint64_t)qi * p.d + i];
+    // the candidates' memory ids in shared memory (one coalesced load)
+    for (uint32_t i = tid; i < cnt; i += NT) {
+        const uint32_t mi = tags[i];
+        stag[i] = mi;
+        if (PQ) {  // the candidates' rows are on their way while the table is built
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(p.pq_codes + (uint64_t)mi * p.pq_code_stride));
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(p.pq_offsets + mi));
+        }
     }
+    tags = stag;
     __syncthreads();
+    if (PQ && p.pq_table) {
+        if (p.pq_lsq == 1) {  // entries (q_m - c)^2: l2sqr_sse of one dimension
+            const float4* cb4 = reinterpret_cast<const float4*>(p.pq_codebook);
+#pragma unroll 4
+            for (uint32_t e = tid; e < p.pq_nsq * 64; e += NT) {
+                const float4 c = __ldg(cb4 + e);
+                const float x = qv[e >> 6];
+                const float d0 = __fsub_rn(x, c.x), d1 = __fsub_rn(x, c.y);
+                const float d2 = __fsub_rn(x, c.z), d3 = __fsub_rn(x, c.w);
+                reinterpret_cast<float4*>(pq_lut)[e] = make_float4(
+                    __fmul_rn(d0, d0), __fmul_rn(d1, d1), __fmul_rn(d2, d2), __fmul_rn(d3, d3));
+            }
+        } else {
+            for (uint32_t e = tid; e < p.pq_nsq * 256; e += NT)
+                pq_lut[e] = l2sqr_sse(qv + (e >> 8) * p.pq_lsq,
+                                      p.pq_codebook + (uint64_t)e * p.pq_lsq, p.pq_lsq);
+        }
+        __syncthreads();
+    }
     if (PQ) {
         const float qn = p.qnorm[qi];
         const float* hd = p.hdist + (uint64_t)qi * p.T;
-        if (p.pq_lsq == 1) {
-            // one-dimensional subspaces: each table entry (q_m - c)^2 is formed when
-            // it is looked up (one subtraction, one product: the same bits as the
-            // table), summed in lookup_dist_table's lane order
-            for (uint32_t j = tid; j < cnt; j += kThreads) {
-                const uint32_t mi = tags[j];
-                const uint32_t* w = reinterpret_cast<const uint32_t*>(
-                    p.pq_codes + (uint64_t)mi * p.pq_code_stride);
+        const bool wide = ((p.pq_code_stride | p.pq_nsq) & 15u) == 0;
+        auto start = [&](uint32_t j) {
+            return __fadd_rn(__fsub_rn(hd[j], qn), __ldg(p.pq_offsets + tags[j]));
+        };
+        auto row = [&](uint32_t j) { return p.pq_codes + (uint64_t)tags[j] * p.pq_code_stride; };
+        if (p.pq_table && wide && !p.pq_sequential) {
+            // rows of whole 16-byte words; lookup_dist_table's order, 16 entries at a time
+            for (uint32_t j = tid; j < cnt; j += NT) {
+                const uint4* w = reinterpret_cast<const uint4*>(row(j));
+                const float t = start(j);
                 float a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                float t = __fadd_rn(__fsub_rn(hd[j], qn), p.pq_offsets[mi]);
+                uint4 c = __ldg(w);
+                const float* col = pq_lut;
+                for (uint32_t m0 = 0; m0 < p.pq_nsq; m0 += 16, col += 16 * 256) {
+                    const uint32_t cw[4] = {c.x, c.y, c.z, c.w};
+                    if (m0 + 16 < p.pq_nsq) c = __ldg(w + (m0 >> 4) + 1);
+                    float x[16];
+#pragma unroll
+                    for (int k = 0; k < 16; ++k)
+                        x[k] = col[k * 256 + ((cw[k >> 2] >> (8 * (k & 3))) & 255u)];
+#pragma unroll
+                    for (int k = 0; k < 16; ++k) a[k & 3] = __fadd_rn(a[k & 3], x[k]);
+                }
+                dist[j] = __fadd_rn(t, __fadd_rn(__fadd_rn(a[0], a[1]), __fadd_rn(a[2], a[3])));
+            }
+        } else if (p.pq_table) {
+            for (uint32_t j = tid; j < cnt; j += NT) {
+                const uint8_t* code = row(j);
+                float t = start(j);
+                if (p.pq_sequential) {
+                    for (uint32_t m = 0; m < p.pq_nsq; ++m)
+                        t = __fadd_rn(t, pq_lut[m * 256 + code[m]]);
+                } else {
+                    t = __fadd_rn(t, lut_sum(code, pq_lut, p.pq_nsq));
+                }
+                dist[j] = t;
+            }
+        } else {
+            // one-dimensional subspaces whose table does not fit: each entry (q_m - c)^2 is
+            // formed when it is looked up (the same bits), in the same order
+            for (uint32_t j = tid; j < cnt; j += NT) {
+                const uint32_t* w = reinterpret_cast<const uint32_t*>(row(j));
+                float a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                float t = start(j);
                 for (uint32_t m0 = 0; m0 < p.pq_nsq; m0 += 4) {
                     const uint32_t c4 = __ldg(w + (m0 >> 2));
 #pragma unroll
@@ -296,28 +399,10 @@ __global__ __launch_bounds__(kThreads) void k_rerank(RerankParams p) {
                     t = __fadd_rn(t, __fadd_rn(__fadd_rn(a[0], a[1]), __fadd_rn(a[2], a[3])));
                 dist[j] = t;
             }
-        } else {
-            for (uint32_t e = tid; e < p.pq_nsq * 256; e += kThreads)
-                pq_lut[e] = l2sqr_sse(qv + (e >> 8) * p.pq_lsq,
-                                      p.pq_codebook + (uint64_t)e * p.pq_lsq, p.pq_lsq);
-            __syncthreads();
-            for (uint32_t j = tid; j < cnt; j += kThreads) {
-                const uint32_t mi = tags[j];
-                float t = __fsub_rn(hd[j], qn);
-                t = __fadd_rn(t, p.pq_offsets[mi]);
-                const uint8_t* code = p.pq_codes + (uint64_t)mi * p.pq_code_stride;
-                if (p.pq_sequential) {
-                    for (uint32_t m = 0; m < p.pq_nsq; ++m)
-                        t = __fadd_rn(t, pq_lut[m * 256 + code[m]]);
-                } else {
-                    t = __fadd_rn(t, lut_sum(code, pq_lut, p.pq_nsq));
-                }
-                dist[j] = t;
-            }
         }
     }
     // kRows rows per warp with their loads in flight together
-    for (uint32_t j0 = warp * kRows; !PQ && j0 < cnt; j0 += kWarps * kRows) {
+    for (uint32_t j0 = warp * kRows; !PQ && j0 < cnt; j0 += (NT / 32) * kRows) {
         const float* rows[kRows];
 #pragma unroll
         for (int u = 0; u < kRows; ++u) {
@@ -338,10 +423,10 @@ __global__ __launch_bounds__(kThreads) void k_rerank(RerankParams p) {
     // (topk+1)-th smallest distance (ties included) and sort just those.
     uint32_t m2 = p.Tp;
     if (cnt > topk + 1) {
-        const float U = key_to_float(block_kth_key<kThreads>(dist, cnt, topk + 1, sel_hist, sel_state));
+        const float U = key_to_float(block_kth_key<NT>(dist, cnt, topk + 1, sel_hist, sel_state));
         if (tid == 0) sel_count = 0;
         __syncthreads();
-        for (uint32_t i = tid; i < cnt; i += kThreads)
+        for (uint32_t i = tid; i < cnt; i += NT)
             if (dist[i] <= U) {
                 const uint32_t pos = atomicAdd(&sel_count, 1u);
                 sv[pos] = dist[i];
@@ -351,12 +436,12 @@ __global__ __launch_bounds__(kThreads) void k_rerank(RerankParams p) {
         const uint32_t m = sel_count;
         m2 = 2;
         while (m2 < m) m2 <<= 1;
-        for (uint32_t i = m + tid; i < m2; i += kThreads) {
+        for (uint32_t i = m + tid; i < m2; i += NT) {
             sv[i] = __int_as_float(0x7f800000);
             si[i] = 0xFFFFFFFFu;
         }
     } else {
-        for (uint32_t i = tid; i < p.Tp; i += kThreads) {
+        for (uint32_t i = tid; i < p.Tp; i += NT) {
             sv[i] = i < cnt ? dist[i] : __int_as_float(0x7f800000);
             si[i] = i < cnt ? i : 0xFFFFFFFFu;
         }
@@ -364,7 +449,7 @@ __global__ __launch_bounds__(kThreads) void k_rerank(RerankParams p) {
     __syncthreads();
     for (uint32_t size = 2; size <= m2; size <<= 1) {
         for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-            for (uint32_t t = tid; t < m2 / 2; t += kThreads) {
+            for (uint32_t t = tid; t < m2 / 2; t += NT) {
                 const uint32_t lo = 2 * t - (t & (stride - 1));
                 const uint32_t hi = lo + stride;
                 const bool asc = (lo & size) == 0;
@@ -386,11 +471,11 @@ __global__ __launch_bounds__(kThreads) void k_rerank(RerankParams p) {
     // anywhere among the results when there are no more candidates than topk
     const uint32_t check = cnt <= topk ? (cnt > 0 ? cnt - 1 : 0) : topk;
     int tie = 0;
-    for (uint32_t i = tid; i < check; i += kThreads)
+    for (uint32_t i = tid; i < check; i += NT)
         if (sv[i] == sv[i + 1]) tie = 1;
     tie = __syncthreads_or(tie);
     if (!tie) {
-        for (uint32_t i = tid; i < topk; i += kThreads) {
+        for (uint32_t i = tid; i < topk; i += NT) {
             od[i] = i < keep ? sv[i] : sentinel_f();
             oi[i] = i < keep ? p.mem2local[tags[si[i]]] : kNoLabel;
         }
@@ -398,25 +483,11 @@ __global__ __launch_bounds__(kThreads) void k_rerank(RerankParams p) {
     }
     __syncthreads();
     if (p.sort_ties)
-        order_by_filter_key<kThreads>(p.hdist + (uint64_t)qi * p.T, tags, cnt, p.Tp, okey, opos);
-    if (tid == 0) {
-        // exact MaxHeap(topk) replay in candidate order, then reorder()
-        float* hv = sv - 1;
-        uint32_t* ht = si - 1;
-        for (uint32_t i = 1; i <= topk; ++i) hv[i] = sentinel_f();
-        uint32_t dpc = topk;
-        for (uint32_t r = 0; r < cnt; ++r) {
-            const uint32_t j = p.sort_ties ? opos[r] : r;
-            const float v = dist[j];
-            if (v < hv[1]) heap_update(hv, ht, topk, dpc, v, p.mem2local[tags[j]]);
-        }
-        heap_reorder(hv, ht, topk);
-        const uint32_t rn = topk - dpc;
-        for (uint32_t i = 0; i < topk; ++i) {
-            od[i] = hv[i + 1];
-            oi[i] = i < rn ? ht[i + 1] : kNoLabel;
-        }
-    }
+        order_by_filter_key<NT>(p.hdist + (uint64_t)qi * p.T, tags, cnt, p.Tp, okey, opos);
+    // (the sort keys are no longer read)
+    if (warp == 0)
+        heap_replay(reinterpret_cast<uint2*>(okey), dist, p.sort_ties ? opos : nullptr, cnt, topk, tags,
+                    p.mem2local, od, oi);
 }
 
 // Bound on |d~ - d| for a row with |x| <= xabs and screened distance d~ (d dims).
@@ -451,9 +522,7 @@ __global__ __launch_bounds__(kScreenThreads, PGPU_RERANK_SCREEN_MIN_BLOCKS) void
     float* approx = qv + p.d;                                                // [T]
     float* hi = approx + p.T;                                                // [T] d~ + E, then exact
     float* bnd = hi + p.T;                                                   // [T]
-    float* hv = bnd + p.T;                                                   // [topk + 1]
-    uint32_t* ht = reinterpret_cast<uint32_t*>(hv + p.topk + 1);             // [topk + 1]
-    uint32_t* opos = ht + p.topk + 1;                                        // [Tp]
+    uint32_t* opos = reinterpret_cast<uint32_t*>(bnd + p.T);                 // [Tp]
     __shared__ uint32_t hist[256];
     __shared__ uint32_t state[2];
     __shared__ uint32_t wcount;
@@ -640,22 +709,8 @@ __global__ __launch_bounds__(kScreenThreads, PGPU_RERANK_SCREEN_MIN_BLOCKS) void
     __syncthreads();
     // the heap is fed in the filter's (t, memory id) order
     order_by_filter_key<kScreenThreads>(p.hdist + (uint64_t)qi * p.T, tags, cnt, p.Tp, keys, opos);
-    if (tid == 0) {
-        float* h1 = hv;  // 1-based: slots 1..topk
-        for (uint32_t i = 1; i <= topk; ++i) h1[i] = sentinel_f();
-        uint32_t dpc = topk;
-        for (uint32_t r = 0; r < cnt; ++r) {
-            const uint32_t j = opos[r];
-            const float v = hi[j];
-            if (v < h1[1]) heap_update(h1, ht, topk, dpc, v, p.mem2local[tags[j]]);
-        }
-        heap_reorder(h1, ht, topk);
-        const uint32_t rn = topk - dpc;
-        for (uint32_t i = 0; i < topk; ++i) {
-            od[i] = h1[i + 1];
-            oi[i] = i < rn ? ht[i + 1] : kNoLabel;
-        }
-    }
+    if (warp == 0)
+        heap_replay(reinterpret_cast<uint2*>(keys), hi, opos, cnt, topk, tags, p.mem2local, od, oi);
 }
 
 uint32_t pow2_at_least(uint32_t v) {
@@ -666,6 +721,7 @@ uint32_t pow2_at_least(uint32_t v) {
 
 }  // namespace
 
+// The limit on filter_topk and topk is checked against this size (the launch may take less).
 size_t rerank_smem_bytes(const DeviceIndex& ix, uint32_t T, uint32_t topk) {
     const uint32_t Tp = pow2_at_least(T > topk ? T : topk);
     // the PQ table is only held for subspaces of more than one dimension
@@ -702,10 +758,18 @@ cudaError_t launch_rerank(const DeviceIndex& ix, const SearchConfig& cfg, uint32
     p.T = s.T;
     p.Tp = pow2_at_least(s.T > topk ? s.T : topk);
     p.topk = topk;
-    const size_t smem = rerank_smem_bytes(ix, s.T, topk);
+    // the sort arrays, or the PQ table while the distances are formed; then query, distances
+    // and ids. The table of one-dimensional subspaces is left out where it does not fit.
+    const size_t sort = (sizeof(float) + 2 * sizeof(uint32_t) + 8) * (size_t)p.Tp;
+    const size_t table = sizeof(float) * 256 * (size_t)ix.pq_nsq;
+    const size_t rest = sizeof(float) * (ix.d + (size_t)s.T) + sizeof(uint32_t) * (size_t)s.T;
+    p.pq_table = ix.pq_nsq && (ix.pq_lsq > 1 || table + rest + 16 <= 220 * 1024);
+    const size_t work = p.pq_table && table > sort ? table : sort;
+    p.work_bytes = (uint32_t)((work + 15) / 16 * 16);
+    const size_t smem = p.work_bytes + rest;
     if (ix.pq_nsq) {
         ensure_max_dynamic_smem(k_rerank<true>, 220 * 1024);
-        k_rerank<true><<<n, kThreads, smem, stream>>>(p);
+        k_rerank<true><<<n, kPqThreads, smem, stream>>>(p);
     } else {
         ensure_max_dynamic_smem(k_rerank<false>, 220 * 1024);
         k_rerank<false><<<n, kThreads, smem, stream>>>(p);

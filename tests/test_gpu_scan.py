@@ -2,7 +2,8 @@
 paths change hands: every record kept or a sampled bound, buffers that overflow and
 queries with more clusters than slots (both answered by the fused kernel), filter_topk
 of 1, above the buffer of two blocks per SM, and above the records of the probed
-clusters; rows of cell terms that are not whole float4s; groups of clusters.
+clusters; rows of cell terms that are not whole float4s; groups of clusters. Then the rerank
+of both modes: forms of the PQ table, and equal distances, whose order is the heap's.
 """
 import os
 import tempfile
@@ -24,18 +25,20 @@ def _lib():
     native.load(build_if_missing=True)
 
 
-def _index(tmp, n, d, C, F, nsq, seed, distinct):
+def _index(tmp, n, d, C, F, nsq, seed, distinct, pq_nsq=0):
     import torch
     from puck_gb300 import builder
     base = builder.gmm(n, d, 64, "unit", seed)
     if distinct:
         base = base[torch.arange(n, device=base.device) % distinct].contiguous()
     a = builder.build_index(base, C, F, nsq, False, train_sample=min(n, 65536), iters=4,
-                            pq_sample=min(n, 32768), seed=seed)
+                            pq_sample=min(n, 32768), seed=seed, whether_pq=pq_nsq > 0,
+                            pq_nsq=pq_nsq or None)
     index_io.write_index(tmp, base=a["base"], coarse=a["coarse"], fine=a["fine"],
                          cell_assign=a["cell_assign"], filter_codebook=a["filter_codebook"],
                          filter_offsets=a["filter_offsets"], filter_codes=a["filter_codes"],
-                         whether_norm=False)
+                         whether_norm=False, pq_codebook=a.get("pq_codebook"),
+                         pq_offsets=a.get("pq_offsets"), pq_codes=a.get("pq_codes"))
     return builder.gmm(70, d, 64, "unit", seed, row_seed=seed + 7).cpu().numpy()
 
 
@@ -59,6 +62,33 @@ def test_scan_matches_oracle(n, d, C, F, nsq, P, T, distinct):
         dist, ids = ix.search(q, k)
         od, oi, st = oracle.OracleIndex(tmp).search_batch(q, k, P, T, topk_max=k,
                                                           nthreads=os.cpu_count(), scan=True)
+        assert (st == 0).all()
+        assert np.array_equal(dist.view(np.uint32), od.view(np.uint32))
+        assert np.array_equal(ids, oi)
+
+
+@pytest.mark.parametrize("mode", [native.PGPU_MODE_EXACT, native.PGPU_MODE_SCAN])
+@pytest.mark.parametrize("d,nsq,pq_nsq,T,k,distinct", [
+    (64, 16, 64, 300, 10, 0),     # table of one-dimensional subspaces, whole 16-byte rows
+    (36, 12, 36, 513, 100, 0),    # rows that are not
+    (96, 24, 48, 200, 10, 0),     # subspaces of two dimensions
+    (192, 24, 192, 3600, 10, 0),  # a table too large for shared memory (exact mode)
+    (32, 8, 32, 1100, 100, 300),  # equal distances: the heap's own order, PQ
+    (32, 8, 0, 700, 100, 200),    # and on the vectors
+    (32, 8, 0, 65, 64, 40),       # a heap of as many as the candidates allow
+    (30, 6, 0, 40, 1, 25),        # and of one
+])
+def test_rerank_matches_oracle(d, nsq, pq_nsq, T, k, distinct, mode):
+    P = 6
+    if mode == native.PGPU_MODE_SCAN:
+        T = min(T, 2048)  # the scan's largest
+    with tempfile.TemporaryDirectory() as tmp:
+        q = _index(tmp, 20_000, d, 10, 24, nsq, 9, distinct, pq_nsq)
+        ix = native.GpuIndex(tmp, search_coarse_count=P, filter_topk=T, topk=k, max_batch=64, mode=mode)
+        dist, ids = ix.search(q, k)
+        od, oi, st = oracle.OracleIndex(tmp).search_batch(q, k, P, T, topk_max=k,
+                                                          nthreads=os.cpu_count(),
+                                                          scan=mode == native.PGPU_MODE_SCAN)
         assert (st == 0).all()
         assert np.array_equal(dist.view(np.uint32), od.view(np.uint32))
         assert np.array_equal(ids, oi)

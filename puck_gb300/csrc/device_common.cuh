@@ -18,6 +18,23 @@ __device__ __forceinline__ float dot_seq(const float* x, const float* y, uint32_
     return s;
 }
 
+// The same sum over a row y in device memory: 16-byte loads where it allows them (one load
+// instruction of a warp whose lanes hold different rows costs a cycle per row, whatever its
+// width).
+__device__ __forceinline__ float dot_seq_row(const float* x, const float* __restrict__ y, uint32_t n) {
+    if ((n & 3u) != 0 || (reinterpret_cast<uintptr_t>(y) & 15u) != 0) return dot_seq(x, y, n);
+    float s = 0.0f;
+#pragma unroll 8
+    for (uint32_t i = 0; i < n; i += 4) {
+        const float4 b = __ldg(reinterpret_cast<const float4*>(y + i));
+        s = __fadd_rn(s, __fmul_rn(x[i], b.x));
+        s = __fadd_rn(s, __fmul_rn(x[i + 1], b.y));
+        s = __fadd_rn(s, __fmul_rn(x[i + 2], b.z));
+        s = __fadd_rn(s, __fmul_rn(x[i + 3], b.w));
+    }
+    return s;
+}
+
 // ------------------------------------------------------------------ MaxHeap
 // Puck's bounded max-heap (puck/hierarchical_cluster/max_heap.cpp:28-102) on
 // 1-based arrays: reject v >= top; the first `size` inserts sift down from the
@@ -137,6 +154,47 @@ __device__ inline void warp_heap_reorder(uint2* heap, uint32_t size, const HeapL
         if ((threadIdx.x & 31) == 0) heap[hs] = top;
         __syncwarp();
     }
+}
+
+// MaxHeap(K) fed with n values in the given order (null: as they are), tags their places,
+// then reorder(), by one warp: heap[1..K], K + 2 entries, 16-byte aligned. Returns the slots
+// filled. A ballot finds the next value below the top, so the steps are the insertions, about
+// K (1 + ln(n / K)) of them, and not the values; the first K / 2 land in leaves, at once.
+__device__ __forceinline__ uint32_t warp_heap_replay(uint2* heap, const float* v,
+                                                     const uint32_t* order, uint32_t n, uint32_t K) {
+    const uint32_t lane = threadIdx.x & 31;
+    const HeapLane hl = heap_lane();
+    for (uint32_t i = lane; i < K + 2; i += 32) heap[i] = make_uint2(__float_as_uint(sentinel_f()), 0u);
+    __syncwarp();
+    float top = sentinel_f();
+    uint32_t dpc = K;
+    for (uint32_t r0 = 0; r0 < n; r0 += 32) {
+        const uint32_t r = r0 + lane;
+        const uint32_t j = r < n ? (order ? order[r] : r) : 0u;
+        const float x = r < n ? v[j] : sentinel_f();
+        unsigned todo = __ballot_sync(0xffffffffu, r < n && x < top);
+        if (dpc > K / 2 && dpc > 1) {  // leaves: the top does not change
+            const uint32_t leaves = dpc - (K / 2 > 1 ? K / 2 : 1u);
+            const uint32_t rank = __popc(todo & ((1u << lane) - 1));
+            const bool leaf = (todo >> lane & 1u) && rank < leaves;
+            if (leaf) heap[dpc - rank] = make_uint2(__float_as_uint(x), j);
+            __syncwarp();
+            const unsigned done = __ballot_sync(0xffffffffu, leaf);
+            dpc -= __popc(done);
+            todo &= ~done;
+        }
+        while (todo) {
+            const int src = __ffs(todo) - 1;
+            const uint32_t f = dpc > 0 ? dpc-- : 1u;
+            const float landed = warp_heap_insert(heap, K, f, __shfl_sync(0xffffffffu, x, src),
+                                                  __shfl_sync(0xffffffffu, j, src), hl);
+            if (f == 1) top = landed;
+            // later values, still below the top
+            todo = __ballot_sync(0xffffffffu, (todo >> lane & 1u) && (int)lane > src && x < top);
+        }
+    }
+    warp_heap_reorder(heap, K, hl);
+    return K - dpc;
 }
 
 // ------------------------------------------------------------- block scans

@@ -174,11 +174,12 @@ __global__ void k_cell_constants(float* __restrict__ stationary, const uint32_t*
 
 // Per row: ascending order of L values by (value, index); the first K are
 // written out. Equal to Puck's heap + reorder() whenever no two values among the
-// first K+1 are equal; otherwise one thread replays the heap exactly.
+// first K+1 are equal; otherwise one warp replays the heap exactly (a thread took half a
+// millisecond over a thousand values, and held up the launch).
 __global__ void k_topsort(const float* __restrict__ vals, uint32_t L, uint32_t Lp, uint32_t ld,
                           uint32_t K, float* __restrict__ out_val, uint32_t* __restrict__ out_idx,
                           const int32_t* __restrict__ status) {
-    extern __shared__ unsigned char smem[];
+    extern __shared__ __align__(16) unsigned char smem[];
     float* sv = reinterpret_cast<float*>(smem);
     uint32_t* si = reinterpret_cast<uint32_t*>(sv + Lp);
     const uint32_t row = blockIdx.x;
@@ -228,19 +229,13 @@ __global__ void k_topsort(const float* __restrict__ vals, uint32_t L, uint32_t L
         }
         return;
     }
-    if (threadIdx.x == 0) {
-        // Exact replay of MaxHeap(K) fed in index order, then reorder().
-        float* hv = sv - 1;
-        uint32_t* ht = si - 1;
-        for (uint32_t i = 1; i <= K; ++i) hv[i] = sentinel_f();
-        uint32_t dpc = K;
-        for (uint32_t i = 0; i < L; ++i) heap_update(hv, ht, K, dpc, v[i], i);
-        heap_reorder(hv, ht, K);
-    }
+    // Exact replay of MaxHeap(K) fed in index order, then reorder(), by one warp.
+    uint2* heap = reinterpret_cast<uint2*>(smem);  // [K + 2]
+    if (threadIdx.x < 32) warp_heap_replay(heap, v, nullptr, L, K);
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < K; i += blockDim.x) {
-        ov[i] = sv[i];
-        oi[i] = si[i];
+        ov[i] = __uint_as_float(heap[i + 1].x);
+        oi[i] = heap[i + 1].y;
     }
 }
 
@@ -520,7 +515,7 @@ cudaError_t launch_topsort_status(const float* vals, uint32_t nrows, uint32_t L,
         return cudaGetLastError();
     }
     const uint32_t Lp = next_pow2(L < 2 ? 2 : L);
-    const size_t smem = (size_t)Lp * 8;
+    const size_t smem = (size_t)Lp * 8 + 16;  // the heap of a replay has K + 2 entries
     ensure_max_dynamic_smem(k_topsort, 220 * 1024);
     k_topsort<<<nrows, 512, smem, stream>>>(vals, L, Lp, ld_vals, K, out_val, out_idx, status);
     return cudaGetLastError();

@@ -468,7 +468,7 @@ __global__ __launch_bounds__(kProbeThreads) void k_probe_select(
     for (uint32_t i = tid; i < Pcap; i += kProbeThreads) {
         if (i < np) {
             const uint32_t c = pick[i];
-            cdist[(uint64_t)row * Pcap + i] = __fsub_rn(bias[c], dot_seq(q, cents + (uint64_t)c * d, d));
+            cdist[(uint64_t)row * Pcap + i] = __fsub_rn(bias[c], dot_seq_row(q, cents + (uint64_t)c * d, d));
             ctag[(uint64_t)row * Pcap + i] = c;
         } else {
             cdist[(uint64_t)row * Pcap + i] = sentinel_f();

@@ -229,37 +229,14 @@ __device__ __forceinline__ void rows8_l2_exact(const float* const* rows, const f
 }
 
 // The exact MaxHeap(topk) fed with cnt distances in the given order (null: as they are), then
-// reorder(), written out; by one warp. heap: topk + 2 entries, 16-byte aligned. A ballot
-// finds the next distance below the top, so the steps are the insertions (about
-// topk (1 + ln(cnt / topk)) of them) and not the candidates; one thread doing all, with each
-// tag fetched from memory, took 0.2 ms for 1100 candidates and topk 100 (a query in that
-// path ended a whole batch's launch).
+// reorder(), written out; by one warp (heap: topk + 2 entries, 16-byte aligned). One thread
+// doing all, with each tag fetched from memory, took 0.2 ms for 1100 candidates and topk 100
+// (a query in that path ended a whole batch's launch).
 __device__ __noinline__ void heap_replay(uint2* heap, const float* dist, const uint32_t* order,
                                          uint32_t cnt, uint32_t topk, const uint32_t* tags,
                                          const uint32_t* mem2local, float* od, uint32_t* oi) {
-    const uint32_t lane = threadIdx.x & 31;
-    const HeapLane hl = heap_lane();
-    for (uint32_t i = lane; i < topk + 2; i += 32) heap[i] = make_uint2(__float_as_uint(sentinel_f()), 0u);
-    __syncwarp();
-    float top = sentinel_f();
-    uint32_t dpc = topk;
-    for (uint32_t r0 = 0; r0 < cnt; r0 += 32) {
-        const uint32_t r = r0 + lane;
-        const uint32_t j = r < cnt ? (order ? order[r] : r) : 0u;
-        const float v = r < cnt ? dist[j] : sentinel_f();
-        unsigned todo = __ballot_sync(0xffffffffu, r < cnt && v < top);
-        while (todo) {
-            const int src = __ffs(todo) - 1;
-            warp_heap_insert(heap, topk, dpc > 0 ? dpc-- : 1u, __shfl_sync(0xffffffffu, v, src),
-                             __shfl_sync(0xffffffffu, j, src), hl);
-            top = __uint_as_float(heap[1].x);
-            // later candidates, still below the top
-            todo = __ballot_sync(0xffffffffu, (todo >> lane & 1u) && (int)lane > src && v < top);
-        }
-    }
-    warp_heap_reorder(heap, topk, hl);
-    const uint32_t rn = topk - dpc;
-    for (uint32_t i = lane; i < topk; i += 32) {
+    const uint32_t rn = warp_heap_replay(heap, dist, order, cnt, topk);
+    for (uint32_t i = threadIdx.x & 31; i < topk; i += 32) {
         od[i] = __uint_as_float(heap[i + 1].x);
         oi[i] = i < rn ? mem2local[tags[heap[i + 1].y]] : kNoLabel;
     }

@@ -45,9 +45,8 @@ __global__ __launch_bounds__(kWinThreads) void k_window_topk(
     const uint32_t* __restrict__ nrows_dev) {
     extern __shared__ __align__(16) unsigned char smem[];
     float* shi = reinterpret_cast<float*>(smem);                 // [C]   s^ + E, later exact s
-    float* slo = shi + C;                                        // [C+1] s^ - E, later heap values
-    uint32_t* stag = reinterpret_cast<uint32_t*>(slo + C + 1);   // [C+1] heap tags
-    float* sq = reinterpret_cast<float*>(stag + C + 1);          // [d]
+    float* slo = shi + C;                                        // [C] s^ - E; the heap from here
+    float* sq = slo + 2 * (C + 1);                               // [d]
     unsigned long long* ckey = reinterpret_cast<unsigned long long*>(
         (reinterpret_cast<uintptr_t>(sq + d) + 7) & ~uintptr_t(7));  // [kWinCap]
     __shared__ uint32_t hist[256];
@@ -108,7 +107,7 @@ __global__ __launch_bounds__(kWinThreads) void k_window_topk(
                 if (t < m) {
                     const uint32_t j = (uint32_t)ckey[t];
                     const float v =
-                        __fsub_rn(bias[j], dot_seq(sq, cents + (uint64_t)j * d, d));
+                        __fsub_rn(bias[j], dot_seq_row(sq, cents + (uint64_t)j * d, d));
                     ckey[t] = ((unsigned long long)ordered_key(v) << 32) | j;
                 } else {
                     ckey[t] = ~0ull;
@@ -134,19 +133,18 @@ __global__ __launch_bounds__(kWinThreads) void k_window_topk(
     // Reference path: every exact value, then MaxHeap(P) fed in index order.
     __syncthreads();
     for (uint32_t j = tid; j < C; j += kWinThreads)
-        shi[j] = __fsub_rn(bias[j], dot_seq(sq, cents + (uint64_t)j * d, d));
+        shi[j] = __fsub_rn(bias[j], dot_seq_row(sq, cents + (uint64_t)j * d, d));
     __syncthreads();
-    if (tid == 0) {
-        atomicAdd(fallbacks, 1ull);
-        for (uint32_t i = 1; i <= P; ++i) slo[i] = sentinel_f();
-        uint32_t dpc = P;
-        for (uint32_t j = 0; j < C; ++j) heap_update(slo, stag, P, dpc, shi[j], j);
-        heap_reorder(slo, stag, P);
+    // the heap takes the place of all that follows the values (16-byte aligned)
+    uint2* heap = reinterpret_cast<uint2*>((reinterpret_cast<uintptr_t>(slo) + 15) & ~uintptr_t(15));
+    if (tid < 32) {
+        if (tid == 0) atomicAdd(fallbacks, 1ull);
+        warp_heap_replay(heap, shi, nullptr, C, P);
     }
     __syncthreads();
     for (uint32_t i = tid; i < P; i += kWinThreads) {
-        ov[i] = slo[i + 1];
-        oi[i] = stag[i + 1];
+        ov[i] = __uint_as_float(heap[i + 1].x);
+        oi[i] = heap[i + 1].y;
     }
 }
 
@@ -278,7 +276,7 @@ __global__ __launch_bounds__(256) void k_window_small(
             // together instead of one chunk of the screen at a time
             for (uint32_t i = lane; i < m; i += 32) {
                 const uint32_t j = (uint32_t)keys[i];
-                const float v = __fsub_rn(bias[j], dot_seq(q, cents + (uint64_t)j * d, d));
+                const float v = __fsub_rn(bias[j], dot_seq_row(q, cents + (uint64_t)j * d, d));
                 keys[i] = ((unsigned long long)ordered_key(v) << 32) | j;
             }
             __syncwarp();
@@ -326,7 +324,7 @@ __global__ __launch_bounds__(256) void k_window_small(
     }
     for (uint32_t j0 = 0; j0 < C; j0 += 32) {
         const uint32_t j = j0 + lane;
-        if (j < C) chunk[warp][lane] = __fsub_rn(bias[j], dot_seq(q, cents + (uint64_t)j * d, d));
+        if (j < C) chunk[warp][lane] = __fsub_rn(bias[j], dot_seq_row(q, cents + (uint64_t)j * d, d));
         __syncwarp();
         if (lane == 0) {
             const uint32_t cnt = C - j0 < 32 ? C - j0 : 32;

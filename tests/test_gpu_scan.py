@@ -25,7 +25,7 @@ def _lib():
     native.load(build_if_missing=True)
 
 
-def _index(tmp, n, d, C, F, nsq, seed, distinct, pq_nsq=0):
+def _index(tmp, n, d, C, F, nsq, seed, distinct, pq_nsq=0, equal=False):
     import torch
     from puck_gb300 import builder
     base = builder.gmm(n, d, 64, "unit", seed)
@@ -34,6 +34,9 @@ def _index(tmp, n, d, C, F, nsq, seed, distinct, pq_nsq=0):
     a = builder.build_index(base, C, F, nsq, False, train_sample=min(n, 65536), iters=4,
                             pq_sample=min(n, 32768), seed=seed, whether_pq=pq_nsq > 0,
                             pq_nsq=pq_nsq or None)
+    if equal:
+        for c in (a["coarse"], a["fine"]):
+            c[1::2] = c[0:len(c) - 1:2]
     index_io.write_index(tmp, base=a["base"], coarse=a["coarse"], fine=a["fine"],
                          cell_assign=a["cell_assign"], filter_codebook=a["filter_codebook"],
                          filter_offsets=a["filter_offsets"], filter_codes=a["filter_codes"],
@@ -89,6 +92,23 @@ def test_rerank_matches_oracle(d, nsq, pq_nsq, T, k, distinct, mode):
         od, oi, st = oracle.OracleIndex(tmp).search_batch(q, k, P, T, topk_max=k,
                                                           nthreads=os.cpu_count(),
                                                           scan=mode == native.PGPU_MODE_SCAN)
+        assert (st == 0).all()
+        assert np.array_equal(dist.view(np.uint32), od.view(np.uint32))
+        assert np.array_equal(ids, oi)
+
+
+@pytest.mark.parametrize("C,F,P", [(40, 1, 40), (40, 2, 12), (130, 33, 100), (300, 300, 290)])
+def test_equal_centroids_match_oracle(C, F, P):
+    """Equal coarse and fine scores: the order of the clusters and cells is the heap's."""
+    d, k = 32, 10
+    with tempfile.TemporaryDirectory() as tmp:
+        q = _index(tmp, 12_000, d, C, F, 8, 3, 0, equal=True)
+        ix = native.GpuIndex(tmp, search_coarse_count=P, filter_topk=100, topk=k, max_batch=64,
+                             mode=native.PGPU_MODE_EXACT)
+        dist, ids = ix.search(q, k)
+        assert ix.walk_counters()["coarse_window_fallbacks"] > 0
+        od, oi, st = oracle.OracleIndex(tmp).search_batch(q, k, P, 100, topk_max=k,
+                                                          nthreads=os.cpu_count())
         assert (st == 0).all()
         assert np.array_equal(dist.view(np.uint32), od.view(np.uint32))
         assert np.array_equal(ids, oi)

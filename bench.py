@@ -771,9 +771,7 @@ def run_gpu(args, w, rank, ws):
         else:
             clusters = entry["mean_clusters"] * nq
             # every record of the probed clusters (offset + codes + fine id), the probed
-            # clusters' stationary rows, the query's fine terms and the query; the split
-            # scan's kernel also writes each record's distance (4 B, not counted here:
-            # an intermediate of this design, reported as t_write_bytes)
+            # clusters' stationary rows, the query's fine terms and the query
             byts = recs * (R + 2) + clusters * w["F"] * 4 + nq * w["F"] * 4 + nq * w["d"] * 4
             kern = "k_scan_score"
         # stage 5: the walk, or the scan's record kernel alone
@@ -794,7 +792,7 @@ def run_gpu(args, w, rank, ws):
                 "unit": "GB/s", "frac": round(ach / peak, 5), "traffic": traffic,
                 "peak_source": peak_kind, "algorithmic_bytes_per_launch": int(byts),
                 "kernel_ms": round(ms, 4), "records": int(recs),
-                "t_write_bytes": int(recs * 4) if entry["mode"] == "scan" else 0}
+                "t_write_bytes": 0}  # no distance per record is written
 
     roof = roofline(best, stage, stats, walk_counters)
     plain_roof = roofline(plain_best, plain_stage, plain_stats, plain_counters)

@@ -64,8 +64,7 @@ typedef struct {
     uint32_t filter_topk;
     double radius_rate;
     int32_t device;     /* CUDA device ordinal */
-    uint32_t max_batch; /* queries per device pass; sizes the per-pass scratch (scan mode adds a
-                           distance buffer of 40960 floats per query, 4 MiB to 4 GiB in all) */
+    uint32_t max_batch; /* queries per device pass; sizes the per-pass scratch */
     int32_t mode;       /* PGPU_MODE_* */
     int32_t precision;  /* PGPU_PRECISION_* (default FP32) */
     uint32_t filter_margin; /* BF16 only: extra filter candidates kept for the rerank */

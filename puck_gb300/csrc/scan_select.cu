@@ -2,7 +2,7 @@
 // filter record of its probed coarse clusters (each cluster is one contiguous
 // range in memory order) and keeps the filter_topk smallest ADC distances. Three
 // kernels: the split scan (k_scan_score, "split scan" below), which answers every
-// query whose records fit the per-pass distance buffer; the fused k_scan_il
+// query whose candidates fit its key buffer; the fused k_scan_il
 // (interleaved layout) for the rest; k_scan_select for nsq not a multiple of 4.
 //
 // Per record the distance is the reference's own expression for a scanned point
@@ -29,8 +29,8 @@
 // bin's upper edge. A last exact radix select leaves the set of the filter_topk
 // smallest (t, id) keys, unordered.
 //
-// Blocks start in launch order longest scan first (k_scan_work, k_scan_order),
-// one block per query.
+// Blocks start in launch order longest scan first, queries of neighbouring clusters
+// together (k_scan_work, k_scan_order), one block per query.
 //
 // Precision form (FP16 tables): the table is stored in FP16, scaled per query by a
 // power of two 2^e chosen from the bound (|q| + max |codeword|)^2 >= every entry
@@ -1371,13 +1371,14 @@ __global__ __launch_bounds__(kOrderThreads) void k_scan_order(const uint16_t* __
 // (the compact 2-byte layout costs a shift per lookup, and its smaller footprint buys
 // nothing here).
 //
-// Bound by instruction issue: per record 24 (nsq) lookups of three instructions, and one
-// 128-byte shared-memory wavefront each. With two blocks
-// per SM one block's table and bound overlap the other's records only in part (a block
-// alone does not fill the SM): of a block's 50k SM cycles in 10k queries over 28.8k records
-// of 24 codes each, 33k are the records'. That batch takes 1.63 ms; 2.09 with every
-// distance written out, binned and read back, and 25 us more for the record counts and the
-// fused kernel's idle blocks.
+// Bound by the shared-memory pipe and by issue: per record 24 (nsq) lookups of three
+// instructions and one 128-byte wavefront each (36 cycles per 32 records measured with
+// nothing else, 1.05 ms for the batch below). With two blocks per SM one block's table
+// and bound overlap the other's records only in part (a block alone does not fill the
+// SM): of a block's 50k SM cycles, in 10k queries over 28.8k records of 24 codes each,
+// 33k are the records'. That batch takes 1.63 ms; 2.09 with every distance written out,
+// binned and read back, and 25 us more for the record counts and the fused kernel's idle
+// blocks.
 #ifndef PGPU_SPLIT_REC
 #define PGPU_SPLIT_REC 4
 #endif

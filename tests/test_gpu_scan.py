@@ -25,7 +25,7 @@ def _lib():
     native.load(build_if_missing=True)
 
 
-def _index(tmp, n, d, C, F, nsq, seed, distinct, pq_nsq=0, equal=False):
+def _index(tmp, n, d, C, F, nsq, seed, distinct, pq_nsq=0, equal=False, nq=70):
     import torch
     from puck_gb300 import builder
     base = builder.gmm(n, d, 64, "unit", seed)
@@ -42,7 +42,7 @@ def _index(tmp, n, d, C, F, nsq, seed, distinct, pq_nsq=0, equal=False):
                          filter_offsets=a["filter_offsets"], filter_codes=a["filter_codes"],
                          whether_norm=False, pq_codebook=a.get("pq_codebook"),
                          pq_offsets=a.get("pq_offsets"), pq_codes=a.get("pq_codes"))
-    return builder.gmm(70, d, 64, "unit", seed, row_seed=seed + 7).cpu().numpy()
+    return builder.gmm(nq, d, 64, "unit", seed, row_seed=seed + 7).cpu().numpy()
 
 
 @pytest.mark.parametrize("n,d,C,F,nsq,P,T,distinct", [
@@ -64,6 +64,22 @@ def test_scan_matches_oracle(n, d, C, F, nsq, P, T, distinct):
                              mode=native.PGPU_MODE_SCAN)
         dist, ids = ix.search(q, k)
         od, oi, st = oracle.OracleIndex(tmp).search_batch(q, k, P, T, topk_max=k,
+                                                          nthreads=os.cpu_count(), scan=True)
+        assert (st == 0).all()
+        assert np.array_equal(dist.view(np.uint32), od.view(np.uint32))
+        assert np.array_equal(ids, oi)
+
+
+@pytest.mark.parametrize("n,C,P,distinct", [(60_000, 8, 8, 150), (9_000, 520, 520, 0)])
+def test_fused_kernel_takes_several_queries_per_block(n, C, P, distinct):
+    """Every query left to the fused kernel, and more of them than its blocks: by ties, by
+    clusters (some of them empty)."""
+    with tempfile.TemporaryDirectory() as tmp:
+        q = _index(tmp, n, 32, C, 16, 8, 5, distinct, nq=1400)
+        ix = native.GpuIndex(tmp, search_coarse_count=P, filter_topk=200, topk=10, max_batch=1400,
+                             mode=native.PGPU_MODE_SCAN)
+        dist, ids = ix.search(q, 10)
+        od, oi, st = oracle.OracleIndex(tmp).search_batch(q, 10, P, 200, topk_max=10,
                                                           nthreads=os.cpu_count(), scan=True)
         assert (st == 0).all()
         assert np.array_equal(dist.view(np.uint32), od.view(np.uint32))

@@ -1,6 +1,7 @@
 // Internal types shared by the host loader, the C ABI and the CUDA kernels.
 #pragma once
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdint.h>
 
 #include <string>
@@ -282,6 +283,33 @@ size_t scan_smem_bytes_half(const DeviceIndex& ix, uint32_t T);
 // interleaved layout and its block fits shared memory (the cell terms of F fine clusters,
 // a key buffer well above filter_topk); otherwise the fused kernel answers every query.
 bool scan_split_applies(const DeviceIndex& ix, const Scratch& s);
+// Shared memory of k_scan_score (byte offsets): table, query, slot arrays, cell terms, then the
+// buffer of cap keys (the compact table while the table is built, before them the sampled keys
+// and their select's histogram). bytes 0: no such block.
+struct SplitLayout {
+    uint32_t slots, rows_per, group, srow, keys, cap, bytes;
+};
+SplitLayout split_choice(const DeviceIndex& ix, uint32_t P, uint32_t T);
+constexpr uint32_t kSplitSampleStep = 512;  // records sampled at a time
+constexpr uint32_t kSplitHistKeys = 512;    // key slots the histogram of the sampled keys takes
+// 1-based rank, among S evenly spaced records of N, of the bound for the T smallest: the
+// expected rank S T / N, three and a half standard deviations (four neighbours are sampled
+// together, and neighbours are alike: 2.5 times the variance of independent ones) and three.
+__host__ __device__ inline uint32_t sample_rank(uint32_t S, uint32_t T, uint32_t N) {
+    const float e = (float)S * (float)T / (float)N;
+    return (uint32_t)(e + 3.5f * sqrtf(2.5f * e) + 3.0f);
+}
+// Records sampled of a query's N, for a buffer of cap keys: as many as it takes for the
+// candidates expected to fit it.
+__host__ __device__ inline uint32_t sample_count(uint32_t cap, uint32_t T, uint32_t N) {
+    uint32_t S = kSplitSampleStep;
+    while (S + kSplitSampleStep + kSplitHistKeys <= cap) {
+        const float r = (float)sample_rank(S, T, N), per = (float)N / (float)S;
+        if (r * per + 3.0f * sqrtf(r) * per <= 0.9f * (float)cap && S * 96 >= N) break;
+        S += kSplitSampleStep;
+    }
+    return S;
+}
 // BF16 copy of the vectors and their norms (precision form), synchronous.
 int ensure_bf16_features(DeviceIndex* ix, std::string* err);
 // The precision form's rotated copy of the filter codes (nsq a multiple of 4, at

@@ -1389,11 +1389,6 @@ static_assert(kSplitRec <= 4, "il_bytes has room for steps of 4 blocks");
 constexpr uint32_t kSplitMaxSlots = 512;     // probed clusters a split query may have
 constexpr uint32_t kSplitRows = 4096;        // floats of cell terms a group of clusters may take
 
-// Shared memory: table, query, slot arrays, cell terms, then the keys (the compact table
-// while the table is built, before them the sampled keys and their select's histogram).
-struct SplitLayout {
-    uint32_t slots, rows_per, group, srow, keys, cap, bytes;
-};
 __host__ __device__ inline SplitLayout split_layout(uint32_t nsq, uint32_t d, uint32_t F, uint32_t P,
                                                     uint32_t budget) {
     SplitLayout y;
@@ -1411,8 +1406,13 @@ __host__ __device__ inline SplitLayout split_layout(uint32_t nsq, uint32_t d, ui
     return y;
 }
 // Two blocks per SM when the buffer then takes T keys one and a half times over, else one.
+// Either way the buffer has to take the first sampled keys and their select's histogram.
 constexpr uint32_t kSplitBudget2 = 111 * 1024, kSplitBudget1 = 220 * 1024;
-__host__ __device__ inline uint32_t split_need(uint32_t T) { return T + T / 2 + 512; }
+constexpr uint32_t kSplitLeast = kSplitSampleStep + kSplitHistKeys;
+static uint32_t split_need(uint32_t T) {
+    const uint32_t n = T + T / 2 + 512;
+    return n > kSplitLeast ? n : kSplitLeast;
+}
 
 struct SplitParams {
     const uint32_t* ctag;
@@ -1438,14 +1438,6 @@ struct SplitParams {
     float codebook_max;
     SplitLayout lay;
 };
-
-// 1-based rank, among S evenly spaced records of N, of the bound for the T smallest: the
-// expected rank S T / N, three and a half standard deviations (four neighbours are sampled
-// together, and neighbours are alike: 2.5 times the variance of independent ones) and three.
-__device__ __forceinline__ uint32_t sample_rank(uint32_t S, uint32_t T, uint32_t N) {
-    const float e = (float)S * (float)T / (float)N;
-    return (uint32_t)(e + 3.5f * sqrtf(2.5f * e) + 3.0f);
-}
 
 template <int NSQ, bool HALF>
 __global__ __launch_bounds__(kSplitThreads, 2) void k_scan_score(const __grid_constant__ SplitParams sp) {
@@ -1583,15 +1575,11 @@ __global__ __launch_bounds__(kSplitThreads, 2) void k_scan_score(const __grid_co
     const uint32_t N = sl_start[L];  // records of all probed clusters
     float tau = __int_as_float(0x7f800000);
     if (N > cap) {
-        // the bound, from S sampled records: as many as it takes for the candidates expected
-        // to fit, four or two per thread at a time. Four neighbouring lanes take the records of their
-        // own lanes in one record block: whole sectors, and lookups without bank conflicts.
-        uint32_t S = 2 * NT;
-        while (S + 2 * NT + kHistBins / 2 <= cap) {
-            const float r = (float)sample_rank(S, T, N), per = (float)N / (float)S;
-            if (r * per + 3.0f * sqrtf(r) * per <= 0.9f * (float)cap && S * 96 >= N) break;
-            S += 2 * NT;
-        }
+        // the bound, from S sampled records, four or two per thread at a time. Four neighbouring
+        // lanes take the records of their own lanes in one record block: whole sectors, and
+        // lookups without bank conflicts. The select's histogram follows the S keys.
+        static_assert(kSplitSampleStep == 2 * NT && kSplitHistKeys * 2 == kHistBins, "sample_count");
+        const uint32_t S = sample_count(cap, T, N);
         const float step = (float)N / (float)S;
         auto sample = [&](uint32_t i0, auto count) {
             constexpr int R = decltype(count)::value;
@@ -1936,11 +1924,11 @@ cudaError_t launch_scan_order(const DeviceIndex& ix, uint32_t n, Scratch& s, cud
     return cudaGetLastError();
 }
 
-static SplitLayout split_choice(const DeviceIndex& ix, uint32_t P, uint32_t T) {
+SplitLayout split_choice(const DeviceIndex& ix, uint32_t P, uint32_t T) {
     const SplitLayout two = split_layout(ix.nsq, ix.d, ix.F, P, kSplitBudget2);
     if (two.bytes && two.cap >= split_need(T)) return two;
     const SplitLayout one = split_layout(ix.nsq, ix.d, ix.F, P, kSplitBudget1);
-    return one.bytes && one.cap >= T + 2 * kSplitThreads + 1024 ? one : SplitLayout{};
+    return one.bytes && one.cap >= T + 512 + kSplitLeast ? one : SplitLayout{};
 }
 
 bool scan_split_applies(const DeviceIndex& ix, const Scratch& s) {

@@ -1260,13 +1260,13 @@ __global__ __launch_bounds__(IlShape<HALF>::kThreads, IlShape<HALF>::kMinBlocks)
         }
         if (il_failed) {
             // a copy did not arrive in time: wait (bounded) for every copy issued, so
-            // none lands in shared memory after the block, and report the query as empty
+            // none lands in shared memory after the block, and report this query and
+            // the block's later ones as empty (the rerank reads every count)
             for (uint32_t g = g_done; g < g_issued; ++g) il_wait(bar_of(g), (g / kIlStages) & 1u);
             __syncthreads();
-            if (tid == 0) {
-                p.hcnt[qi] = 0;
-                atomicExch(p.err, 1);
-            }
+            for (uint64_t i = qb + (uint64_t)tid * gridDim.x; i < nq; i += (uint64_t)kIlThreads * gridDim.x)
+                p.hcnt[p.todo ? p.todo[i] : p.order[i]] = 0;
+            if (tid == 0) atomicExch(p.err, 1);
             return;
         }
         scan_finish<kIlThreads>(p, st, keys, hist, qi, my_eval, my_eval, my_pass, t_start, t_pro);

@@ -102,7 +102,7 @@ int check_config(const pgpu_index* h, const pgpu_params* p) {
             (bf16 ? pgpu::scan_smem_bytes_half(h->ix, (uint32_t)keep)
                   : pgpu::scan_smem_bytes(h->ix, (uint32_t)keep)) > 220 * 1024 ||
             (bf16 && h->ix.pq_nsq == 0
-                 ? pgpu::rerank_screen_smem_bytes(h->ix, (uint32_t)keep, p->topk)
+                 ? pgpu::rerank_screen_smem_bytes(h->ix, (uint32_t)keep)
                   : pgpu::rerank_smem_bytes(h->ix, (uint32_t)keep, p->topk)) > 220 * 1024)
             return fail(PGPU_E_LIMIT, "filter_topk/topk/filter_nsq exceed the shared-memory budget");
     }

@@ -315,7 +315,7 @@ int ensure_bf16_features(DeviceIndex* ix, std::string* err);
 // The precision form's rotated copy of the filter codes (nsq a multiple of 4, at
 // most 32; otherwise nothing is made), synchronous.
 int ensure_interleaved_codes(DeviceIndex* ix, std::string* err);
-size_t rerank_screen_smem_bytes(const DeviceIndex& ix, uint32_t T, uint32_t topk);
+size_t rerank_screen_smem_bytes(const DeviceIndex& ix, uint32_t T);
 cudaError_t launch_rerank_screen(const DeviceIndex& ix, uint32_t n, uint32_t topk, const Scratch& s,
                                  float* out_dist, uint32_t* out_ids, int32_t* out_status,
                                  cudaStream_t stream);

@@ -494,8 +494,9 @@ struct ScreenParams {
 
 __global__ __launch_bounds__(kScreenThreads, PGPU_RERANK_SCREEN_MIN_BLOCKS) void k_rerank_screen(ScreenParams p) {
     extern __shared__ __align__(16) unsigned char smem[];
-    unsigned long long* keys = reinterpret_cast<unsigned long long*>(smem);  // [Tp]
-    float* qv = reinterpret_cast<float*>(keys + p.Tp);                       // [d]
+    // [Tp + 2]: a heap replayed here has topk + 2 entries
+    unsigned long long* keys = reinterpret_cast<unsigned long long*>(smem);
+    float* qv = reinterpret_cast<float*>(keys + p.Tp + 2);                   // [d]
     float* approx = qv + p.d;                                                // [T]
     float* hi = approx + p.T;                                                // [T] d~ + E, then exact
     float* bnd = hi + p.T;                                                   // [T]
@@ -754,10 +755,10 @@ cudaError_t launch_rerank(const DeviceIndex& ix, const SearchConfig& cfg, uint32
     return cudaGetLastError();
 }
 
-size_t rerank_screen_smem_bytes(const DeviceIndex& ix, uint32_t T, uint32_t topk) {
+size_t rerank_screen_smem_bytes(const DeviceIndex& ix, uint32_t T) {
     const uint32_t Tp = pow2_at_least(T);
-    return sizeof(unsigned long long) * Tp + sizeof(float) * (ix.d + 3ull * T) +
-           (sizeof(float) + sizeof(uint32_t)) * (topk + 1ull) + sizeof(uint32_t) * (Tp + T);
+    return sizeof(unsigned long long) * (Tp + 2) + sizeof(float) * (ix.d + 3ull * T) +
+           sizeof(uint32_t) * (Tp + T);
 }
 
 cudaError_t launch_rerank_screen(const DeviceIndex& ix, uint32_t n, uint32_t topk, const Scratch& s,
@@ -782,7 +783,7 @@ cudaError_t launch_rerank_screen(const DeviceIndex& ix, uint32_t n, uint32_t top
     p.T = s.T;
     p.Tp = pow2_at_least(s.T);
     p.topk = topk;
-    const size_t smem = rerank_screen_smem_bytes(ix, s.T, topk);
+    const size_t smem = rerank_screen_smem_bytes(ix, s.T);
     ensure_max_dynamic_smem(k_rerank_screen, 220 * 1024);
     k_rerank_screen<<<n, kScreenThreads, smem, stream>>>(p);
     return cudaGetLastError();

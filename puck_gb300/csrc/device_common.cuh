@@ -160,6 +160,8 @@ __device__ inline void warp_heap_reorder(uint2* heap, uint32_t size, const HeapL
 // then reorder(), by one warp: heap[1..K], K + 2 entries, 16-byte aligned. Returns the slots
 // filled. A ballot finds the next value below the top, so the steps are the insertions, about
 // K (1 + ln(n / K)) of them, and not the values; the first K / 2 land in leaves, at once.
+// A value that is not a number enters, as in the heap; SKIP_NAN: it is passed over.
+template <bool SKIP_NAN = false>
 __device__ __forceinline__ uint32_t warp_heap_replay(uint2* heap, const float* v,
                                                      const uint32_t* order, uint32_t n, uint32_t K) {
     const uint32_t lane = threadIdx.x & 31;
@@ -168,11 +170,12 @@ __device__ __forceinline__ uint32_t warp_heap_replay(uint2* heap, const float* v
     __syncwarp();
     float top = sentinel_f();
     uint32_t dpc = K;
+    auto below = [&](float x) { return SKIP_NAN ? x < top : !(x >= top); };
     for (uint32_t r0 = 0; r0 < n; r0 += 32) {
         const uint32_t r = r0 + lane;
         const uint32_t j = r < n ? (order ? order[r] : r) : 0u;
         const float x = r < n ? v[j] : sentinel_f();
-        unsigned todo = __ballot_sync(0xffffffffu, r < n && x < top);
+        unsigned todo = __ballot_sync(0xffffffffu, r < n && below(x));
         if (dpc > K / 2 && dpc > 1) {  // leaves: the top does not change
             const uint32_t leaves = dpc - (K / 2 > 1 ? K / 2 : 1u);
             const uint32_t rank = __popc(todo & ((1u << lane) - 1));
@@ -189,8 +192,8 @@ __device__ __forceinline__ uint32_t warp_heap_replay(uint2* heap, const float* v
             const float landed = warp_heap_insert(heap, K, f, __shfl_sync(0xffffffffu, x, src),
                                                   __shfl_sync(0xffffffffu, j, src), hl);
             if (f == 1) top = landed;
-            // later values, still below the top
-            todo = __ballot_sync(0xffffffffu, (todo >> lane & 1u) && (int)lane > src && x < top);
+            // later values below the top (it only falls, unless no number comes to it)
+            todo = __ballot_sync(0xffffffffu, r < n && (int)lane > src && below(x));
         }
     }
     warp_heap_reorder(heap, K, hl);

@@ -231,11 +231,12 @@ __device__ __forceinline__ void rows8_l2_exact(const float* const* rows, const f
 // The exact MaxHeap(topk) fed with cnt distances in the given order (null: as they are), then
 // reorder(), written out; by one warp (heap: topk + 2 entries, 16-byte aligned). One thread
 // doing all, with each tag fetched from memory, took 0.2 ms for 1100 candidates and topk 100
-// (a query in that path ended a whole batch's launch).
+// (a query in that path ended a whole batch's launch). A distance that is not a number (of a
+// stored vector that is not finite) is no result.
 __device__ __noinline__ void heap_replay(uint2* heap, const float* dist, const uint32_t* order,
                                          uint32_t cnt, uint32_t topk, const uint32_t* tags,
                                          const uint32_t* mem2local, float* od, uint32_t* oi) {
-    const uint32_t rn = warp_heap_replay(heap, dist, order, cnt, topk);
+    const uint32_t rn = warp_heap_replay<true>(heap, dist, order, cnt, topk);
     for (uint32_t i = threadIdx.x & 31; i < topk; i += 32) {
         od[i] = __uint_as_float(heap[i + 1].x);
         oi[i] = i < rn ? mem2local[tags[heap[i + 1].y]] : kNoLabel;

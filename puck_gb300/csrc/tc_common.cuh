@@ -47,6 +47,8 @@ __device__ __forceinline__ float gelu_grad_f(float x) {
     return cdf + x * pdf;
 }
 
+// Tensor maps can be encoded here (the driver offers the call).
+bool tensor_maps_available();
 // 2-D BF16 tensor map of rows x K values at p, rows rs elements apart (16-byte aligned), box
 // 64 (K) x box_rows, 128-byte swizzle, zero fill past the ends.
 bool encode_bf16_rows(CUtensorMap* map, const uint16_t* p, uint64_t rows, uint64_t rs, uint32_t K,

@@ -433,7 +433,8 @@ uint32_t tc_filter_splits(uint32_t M) {
     return mt >= sms ? 1u : sms / mt;
 }
 
-bool tc_filter_applies(uint32_t K) { return K > 0 && K <= kMaxResident * 64; }
+// (without tensor maps nearest_center and knn take the forms with a screen matrix)
+bool tc_filter_applies(uint32_t K) { return K > 0 && K <= kMaxResident * 64 && tensor_maps_available(); }
 
 cudaError_t launch_rows_bf16(const float* X, uint64_t rows, uint32_t d, uint32_t dp, bool seq,
                              uint32_t pad, uint16_t* out, float* norm, float* lost,

@@ -710,6 +710,8 @@ cudaError_t launch_tc_gemm_tma(const TcOperand& A, const TcOperand& B, uint32_t 
 
 }  // namespace
 
+bool tensor_maps_available() { return encode_tiled_fn() != nullptr; }
+
 bool encode_bf16_rows(CUtensorMap* map, const uint16_t* p, uint64_t rows, uint64_t rs, uint32_t K,
                       uint32_t box_rows) {
     EncodeTiledFn fn = encode_tiled_fn();

@@ -7,6 +7,7 @@ import os
 import subprocess
 
 import pytest
+import torch
 
 from puck_gb300 import build, native
 
@@ -35,6 +36,8 @@ def host(tmp_path_factory):
     src.write_text(SOURCE)
     lib = build.build()
     native.load()
+    if torch.cuda.is_available():
+        torch.empty(1, device="cuda")  # the driver encodes once it is initialised
     subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", str(src), "-o", str(so), lib,
                     "-I" + os.path.join(REPO, "puck_gb300", "csrc"),
                     "-I" + os.path.join(build._cuda_home(), "include"), "-Wl,-rpath," + os.path.dirname(lib)],

@@ -580,23 +580,16 @@ int pgpu_knn(const float* base, uint64_t n, uint32_t dim, const float* queries, 
     if (n > 0xFFFFFFFFull) return fail(PGPU_E_LIMIT, "more than 2^32-1 base points");
     if (n == 0 || nq == 0) return PGPU_OK;
     cudaStream_t st = (cudaStream_t)stream;
-    int* flags = nullptr;  // a wait expired, a candidate list overflowed
-    cudaError_t e = cudaMallocAsync(&flags, 2 * sizeof(int), st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(flags, 0, 2 * sizeof(int), st);
-    if (e == cudaSuccess) e = pgpu::launch_knn(base, n, dim, queries, nq, k, labels, distance, flags, st);
-    int got[2] = {0, 0};
-    auto read = [&]() {
-        if (e == cudaSuccess) e = cudaMemcpyAsync(got, flags, sizeof(got), cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    };
-    read();
-    if (e == cudaSuccess && got[1] && !got[0]) {
-        e = pgpu::launch_knn_dense(base, n, dim, queries, nq, k, labels, distance, flags, st);
-        read();
-    }
-    if (flags) cudaFreeAsync(flags, st);
+    int* err = nullptr;
+    cudaError_t e = cudaMallocAsync(&err, sizeof(int), st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(err, 0, sizeof(int), st);
+    if (e == cudaSuccess) e = pgpu::launch_knn(base, n, dim, queries, nq, k, labels, distance, err, st);
+    int flag = 0;
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&flag, err, sizeof(int), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (err) cudaFreeAsync(err, st);
     if (e != cudaSuccess) return cuda_fail(e, "knn");
-    if (got[0]) return fail(PGPU_E_TIMEOUT, "tensor-core wait expired");
+    if (flag) return fail(PGPU_E_TIMEOUT, "tensor-core wait expired");
     return PGPU_OK;
 }
 

@@ -11,12 +11,13 @@
 // The screen's scores are not written out (k_tc_filter): the first kFirst columns go
 // to the queries' lists whole, later ones only where the score is at or below the
 // 64th smallest so far, in growing ranges (a range of twice the columns seen adds
-// about 128 entries per query to a list of 2048). The ranges are spread over
-// the whole base, so that a base in any order adds no more. Should a list overflow
-// all the same, the call is repeated with the screen matrix in memory
-// (launch_knn_dense, which also takes dimensions above the filter's limit).
-// 2048 queries of 96 dimensions over 1M points: 2.1 ms, against 24.5 ms with the screen
-// matrix in memory. The tensor filter's passes are 1.2 ms of it, the lists' merges 0.23.
+// about 128 entries per query to a list of 2048). The ranges are spread over the whole
+// base by tiles of 256 rows. A base in the order of its clusters still puts whole tiles
+// below a query's threshold; the filter cuts a full part of a list back to its 64
+// smallest. Dimensions above the filter's limit: launch_knn_dense, with the screen
+// matrix in memory.
+// 2048 queries of 96 dimensions over 1M points: 2.05 ms (2.7 in the order of their clusters),
+// against 24.5 ms with the screen matrix in memory. The tensor filter's passes are 1.2 ms of it, the lists' merges 0.23.
 #include <algorithm>
 #include <cfloat>
 #include <cstdint>
@@ -29,6 +30,7 @@ namespace pgpu {
 namespace {
 
 constexpr uint32_t kKC = 64;          // candidates per query
+static_assert(kKC <= kTcFilterKeep, "a part keeps all of a query's candidates");
 constexpr int kWarpsPerBlock = 8;
 
 __global__ void k_half_sq_norms(const float* __restrict__ X, uint64_t rows, uint32_t d,
@@ -140,11 +142,11 @@ __global__ __launch_bounds__(kWarpsPerBlock * 32) void k_knn_merge(
 
 // The queries' lists merged into their 64 smallest (score, id), one warp per query; the
 // 64th score becomes the threshold of the next range. A list is `parts` runs of at most
-// seg entries, count[row][part] of them (count null: seg in each).
+// seg entries, count[row][part] <= seg of them (count null: seg in each).
 __global__ __launch_bounds__(kWarpsPerBlock * 32) void k_knn_lists(
     const uint2* __restrict__ cand, uint32_t cap, uint32_t parts, uint32_t seg,
     const uint32_t* __restrict__ count, uint32_t rows, float* __restrict__ cs,
-    uint32_t* __restrict__ ci, float* __restrict__ thr, int* __restrict__ overflow) {
+    uint32_t* __restrict__ ci, float* __restrict__ thr) {
     __shared__ float bv[kWarpsPerBlock][2 * kKC];
     __shared__ uint32_t bi[kWarpsPerBlock][2 * kKC];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -178,10 +180,6 @@ __global__ __launch_bounds__(kWarpsPerBlock * 32) void k_knn_lists(
         // 32 parts' lengths at once
         uint32_t len = 0;
         if (p0 + lane < parts) len = count ? count[(uint64_t)row * parts + p0 + lane] : seg;
-        if (len > seg) {
-            atomicExch(overflow, 1);
-            len = seg;
-        }
         const uint32_t np = parts - p0 < 32 ? parts - p0 : 32;
         // (the loads of two parts are under way while one is merged)
         auto head = [&](uint32_t u) {  // the first entries of part p0 + u
@@ -281,19 +279,69 @@ int rows_vec(const float* a, const float* b, uint32_t d) {
 
 }  // namespace
 
-cudaError_t launch_knn(const float* base, uint64_t n, uint32_t d, const float* Q, uint32_t nq,
-                       uint32_t k, uint32_t* ids, float* dist, int* flags, cudaStream_t st) {
+static cudaError_t launch_knn_dense(const float* base, uint64_t n, uint32_t d, const float* Q,
+                                    uint32_t nq, uint32_t k, uint32_t* ids, float* dist, int* err,
+                                    cudaStream_t st) {
     if (k == 0 || k > kKC || n == 0 || nq == 0) return cudaErrorInvalidValue;
-    if (!tc_filter_applies(d)) return launch_knn_dense(base, n, d, Q, nq, k, ids, dist, flags, st);
+    constexpr uint32_t kQC = 8192, kBC = 16384;
+    float *S = nullptr, *hb = nullptr, *cs = nullptr, *thr = nullptr;
+    uint32_t* ci = nullptr;
+    cudaError_t e = cudaMallocAsync(&S, sizeof(float) * kQC * kBC, st);
+    if (e == cudaSuccess) e = cudaMallocAsync(&hb, sizeof(float) * n, st);
+    if (e == cudaSuccess) e = cudaMallocAsync(&cs, sizeof(float) * kQC * kKC, st);
+    if (e == cudaSuccess) e = cudaMallocAsync(&ci, sizeof(uint32_t) * kQC * kKC, st);
+    if (e == cudaSuccess) e = cudaMallocAsync(&thr, sizeof(float) * kQC, st);
+    if (e == cudaSuccess) {
+        k_half_sq_norms<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(base, n, d, hb);
+        e = cudaGetLastError();
+    }
+    for (uint32_t q0 = 0; e == cudaSuccess && q0 < nq; q0 += kQC) {
+        const uint32_t qr = nq - q0 < kQC ? nq - q0 : kQC;
+        k_knn_reset<<<(qr * kKC + 255) / 256, 256, 0, st>>>(cs, ci, thr, qr);
+        for (uint64_t b0 = 0; e == cudaSuccess && b0 < n; b0 += kBC) {
+            const uint32_t br = (uint32_t)(n - b0 < kBC ? n - b0 : kBC);
+            TcEpilogue ep{};
+            ep.mode = TC_EPI_SCORE;
+            ep.out = S;
+            ep.ld = kBC;
+            ep.bias = hb + b0;
+            e = launch_tc_gemm(TcOperand{Q + (uint64_t)q0 * d, d, 1, qr},
+                               TcOperand{base + b0 * d, d, 1, br}, d, ep, err, st);
+            if (e != cudaSuccess) break;
+            k_knn_merge<<<(qr + kWarpsPerBlock - 1) / kWarpsPerBlock, kWarpsPerBlock * 32, 0, st>>>(
+                S, kBC, qr, br, (uint32_t)b0, cs, ci, thr);
+            e = cudaGetLastError();
+        }
+        if (e != cudaSuccess) break;
+        k_knn_final<<<(qr + kWarpsPerBlock - 1) / kWarpsPerBlock, kWarpsPerBlock * 32, 0, st>>>(
+            base, d, Q + (uint64_t)q0 * d, qr, ci, k, rows_vec(base, Q, d), ids + (uint64_t)q0 * k,
+            dist + (uint64_t)q0 * k);
+        e = cudaGetLastError();
+    }
+    if (S) cudaFreeAsync(S, st);
+    if (hb) cudaFreeAsync(hb, st);
+    if (cs) cudaFreeAsync(cs, st);
+    if (ci) cudaFreeAsync(ci, st);
+    if (thr) cudaFreeAsync(thr, st);
+    return e;
+}
+
+cudaError_t launch_knn(const float* base, uint64_t n, uint32_t d, const float* Q, uint32_t nq,
+                       uint32_t k, uint32_t* ids, float* dist, int* err, cudaStream_t st) {
+    if (k == 0 || k > kKC || n == 0 || nq == 0) return cudaErrorInvalidValue;
+    if (!tc_filter_applies(d)) return launch_knn_dense(base, n, d, Q, nq, k, ids, dist, err, st);
     constexpr uint32_t kQC = 8192, kFirst = 2048 / kTcFilterTile;
     const uint32_t dp = (d + 7u) & ~7u, qc = nq < kQC ? nq : kQC;
-    // list entries per query: 64 at least for each part
-    auto cap_of = [](uint32_t rows) { return std::max(2048u, 128 * tc_filter_splits(rows)); };
-    const uint32_t last = nq % kQC ? nq % kQC : qc;  // rows of the last chunk of queries
     // base rows held in BF16 at a time: 256 MiB, whole tiles
     uint64_t held = (256ull << 20) / (2ull * dp) / kTcFilterTile * kTcFilterTile;
     if (held > n) held = n;
-    const uint64_t padded = (held + kTcFilterTile - 1) / kTcFilterTile * kTcFilterTile;
+    const uint32_t tiles_held = (uint32_t)((held + kTcFilterTile - 1) / kTcFilterTile);
+    const uint64_t padded = (uint64_t)tiles_held * kTcFilterTile;
+    // list entries per query: the first columns, or the least that each part takes
+    auto cap_of = [tiles_held](uint32_t rows) {
+        return std::max(2048u, 2 * kTcFilterPart * std::min(tc_filter_splits(rows), tiles_held));
+    };
+    const uint32_t last = nq % kQC ? nq % kQC : qc;  // rows of the last chunk of queries
     uint64_t bytes = 0;
     auto part = [&](uint64_t size) {
         const uint64_t at = bytes;
@@ -341,7 +389,7 @@ cudaError_t launch_knn(const float* base, uint64_t n, uint32_t d, const float* Q
             p.cand = reinterpret_cast<uint2*>(mem + o_cand);
             p.cap = cap_of(qr);
             p.id0 = (uint32_t)b0;
-            p.err = flags;
+            p.err = err;
             for (uint32_t pos = 0; e == cudaSuccess && pos < tiles;) {
                 const bool first = seen == 0;
                 const uint64_t room = first ? kFirst : 2 * (seen / kTcFilterTile);
@@ -352,7 +400,7 @@ cudaError_t launch_knn(const float* base, uint64_t n, uint32_t d, const float* Q
                 k_knn_lists<<<blocks, kWarpsPerBlock * 32, 0, st>>>(
                     p.cand, p.cap, first ? 1u : 2 * p.splits,
                     first ? (p.pos1 - pos) * kTcFilterTile : p.seg, first ? nullptr : p.count, qr,
-                    f(o_cs), u(o_ci), f(o_thr), flags + 1);
+                    f(o_cs), u(o_ci), f(o_thr));
                 e = cudaGetLastError();
                 seen += (uint64_t)(p.pos1 - pos) * kTcFilterTile;
                 pos = p.pos1;
@@ -364,52 +412,6 @@ cudaError_t launch_knn(const float* base, uint64_t n, uint32_t d, const float* Q
         e = cudaGetLastError();
     }
     cudaFreeAsync(mem, st);
-    return e;
-}
-
-cudaError_t launch_knn_dense(const float* base, uint64_t n, uint32_t d, const float* Q, uint32_t nq,
-                             uint32_t k, uint32_t* ids, float* dist, int* err, cudaStream_t st) {
-    if (k == 0 || k > kKC || n == 0 || nq == 0) return cudaErrorInvalidValue;
-    constexpr uint32_t kQC = 8192, kBC = 16384;
-    float *S = nullptr, *hb = nullptr, *cs = nullptr, *thr = nullptr;
-    uint32_t* ci = nullptr;
-    cudaError_t e = cudaMallocAsync(&S, sizeof(float) * kQC * kBC, st);
-    if (e == cudaSuccess) e = cudaMallocAsync(&hb, sizeof(float) * n, st);
-    if (e == cudaSuccess) e = cudaMallocAsync(&cs, sizeof(float) * kQC * kKC, st);
-    if (e == cudaSuccess) e = cudaMallocAsync(&ci, sizeof(uint32_t) * kQC * kKC, st);
-    if (e == cudaSuccess) e = cudaMallocAsync(&thr, sizeof(float) * kQC, st);
-    if (e == cudaSuccess) {
-        k_half_sq_norms<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(base, n, d, hb);
-        e = cudaGetLastError();
-    }
-    for (uint32_t q0 = 0; e == cudaSuccess && q0 < nq; q0 += kQC) {
-        const uint32_t qr = nq - q0 < kQC ? nq - q0 : kQC;
-        k_knn_reset<<<(qr * kKC + 255) / 256, 256, 0, st>>>(cs, ci, thr, qr);
-        for (uint64_t b0 = 0; e == cudaSuccess && b0 < n; b0 += kBC) {
-            const uint32_t br = (uint32_t)(n - b0 < kBC ? n - b0 : kBC);
-            TcEpilogue ep{};
-            ep.mode = TC_EPI_SCORE;
-            ep.out = S;
-            ep.ld = kBC;
-            ep.bias = hb + b0;
-            e = launch_tc_gemm(TcOperand{Q + (uint64_t)q0 * d, d, 1, qr},
-                               TcOperand{base + b0 * d, d, 1, br}, d, ep, err, st);
-            if (e != cudaSuccess) break;
-            k_knn_merge<<<(qr + kWarpsPerBlock - 1) / kWarpsPerBlock, kWarpsPerBlock * 32, 0, st>>>(
-                S, kBC, qr, br, (uint32_t)b0, cs, ci, thr);
-            e = cudaGetLastError();
-        }
-        if (e != cudaSuccess) break;
-        k_knn_final<<<(qr + kWarpsPerBlock - 1) / kWarpsPerBlock, kWarpsPerBlock * 32, 0, st>>>(
-            base, d, Q + (uint64_t)q0 * d, qr, ci, k, rows_vec(base, Q, d), ids + (uint64_t)q0 * k,
-            dist + (uint64_t)q0 * k);
-        e = cudaGetLastError();
-    }
-    if (S) cudaFreeAsync(S, st);
-    if (hb) cudaFreeAsync(hb, st);
-    if (cs) cudaFreeAsync(cs, st);
-    if (ci) cudaFreeAsync(ci, st);
-    if (thr) cudaFreeAsync(thr, st);
     return e;
 }
 

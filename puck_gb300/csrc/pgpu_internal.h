@@ -357,6 +357,8 @@ cudaError_t launch_tc_gemm(const TcOperand& A, const TcOperand& B, uint32_t K,
                            const TcEpilogue& ep, int* err, cudaStream_t stream);
 // Contraction with a selecting epilogue (tc_filter.cu): s_ij = bias_j - a_i.b_j over BF16 rows.
 constexpr uint32_t kTcFilterTile = 256;  // columns per tile
+constexpr uint32_t kTcFilterKeep = 64;   // BELOW: entries a part keeps when it is cut back
+constexpr uint32_t kTcFilterPart = kTcFilterKeep + 32;  // the least a part takes
 enum { kTcMinima = 0, kTcBelow = 1, kTcDense = 2 };
 struct TcFilter {
     uint32_t M, N, K;          // rows of A and B, dimensions (tc_filter_applies)
@@ -365,7 +367,7 @@ struct TcFilter {
     uint32_t step, tiles;
     float* gmin;               // MINIMA: [M][tiles * 32] smallest score per 8 columns
     const float* thr;          // BELOW: [M] thresholds
-    uint32_t* count;           // BELOW: [M][2 splits] entries of each part (above seg: some lost)
+    uint32_t* count;           // BELOW: [M][2 splits] entries of each part
     uint2* cand;               // (score bits, id0 + column): BELOW [M][2 splits] parts of seg in
                                // rows of cap, DENSE [M][cap] in the order of the positions
     uint32_t cap, id0;
@@ -411,12 +413,9 @@ cudaError_t launch_probe_select(const ProbeNet& net, const DeviceIndex& ix, uint
                                 cudaStream_t st);
 
 // Brute-force kNN on the tensor-core screen with FP32 rescoring (knn.cu); k <= 64.
-// flags (DEVICE): [0] a tensor-core wait expired, [1] a candidate list overflowed: the result
-// is not valid, launch_knn_dense gives it.
+// err (DEVICE): set when a tensor-core wait expired.
 cudaError_t launch_knn(const float* base, uint64_t n, uint32_t d, const float* Q, uint32_t nq,
-                       uint32_t k, uint32_t* ids, float* dist, int* flags, cudaStream_t st);
-cudaError_t launch_knn_dense(const float* base, uint64_t n, uint32_t d, const float* Q, uint32_t nq,
-                             uint32_t k, uint32_t* ids, float* dist, int* err, cudaStream_t st);
+                       uint32_t k, uint32_t* ids, float* dist, int* err, cudaStream_t st);
 const ProbeNet* probe_net(const pgpu_probe* p);
 int probe_device(const pgpu_probe* p);
 

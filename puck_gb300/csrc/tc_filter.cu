@@ -8,7 +8,10 @@
 //   BELOW   the (score, column) pairs at or below a row's threshold, in its list: the screen of
 //           the brute-force neighbours. A row's list has a part for each warp that works on the
 //           row, so an entry costs no atomic (one with its result on the way took 3 of the 6 ms
-//           of a million columns). DENSE fills the lists for the first columns.
+//           of a million columns). A part that may not take 32 more columns' entries is cut
+//           back to its kTcFilterKeep smallest, which are all that the row's smallest can need of it, and
+//           the last of them is the row's threshold there: no order of the columns overflows a
+//           list. DENSE fills the lists for the first columns.
 //
 // One CTA per SM loops over items, an item being a 128-row tile of A and every splits-th of a
 // range of 256-column tiles of B (position p stands for tile (p * step) mod tiles: a range of
@@ -46,6 +49,65 @@ constexpr uint32_t kABytes = 128u * 64u * 2u, kBBytes = kNT * 64u * 2u;
 
 // A tiles held: two where they fit beside the ring.
 __host__ __device__ constexpr uint32_t a_buffers(uint32_t nch) { return nch <= 2 ? 2u : 1u; }
+
+// A part of a list cut back to its kTcFilterKeep smallest (score, column), by one warp: kept keys
+// sorted in registers (0 and 1; two per lane), the rest brought in 64 at a time (2 and 3) and the
+// 128 sorted. Returns the largest score kept. n > kTcFilterKeep entries. Asked for after every 32
+// columns, so that a part needs room for 96 entries and no more memory than without: one million
+// rows in the order of 1024 clusters, 2048 queries, take 2.7 ms (28 where an overflowing part had
+// the call repeated with the screen in memory), shuffled 2.16 (2.23). Asked after 128 columns
+// the larger parts cost 30 to 90 us of allocation; one thread replacing the largest of its full
+// part took 9.3 ms.
+__device__ __noinline__ float cut_back(uint2* list, uint32_t n) {
+    static_assert(kTcFilterKeep == 64, "two keys per lane");
+    const uint32_t lane = threadIdx.x & 31;
+    __syncwarp();  // the lane that wrote the entries is another
+    unsigned long long a[4];
+    auto fetch = [&](uint32_t i) {
+        if (i >= n) return ~0ull;
+        const uint2 e = list[i];
+        return ((unsigned long long)ordered_key(__uint_as_float(e.x) + 0.0f) << 32) | e.y;  // -0 is 0
+    };
+    a[0] = fetch(lane);
+    a[1] = fetch(lane + 32);
+    for (uint32_t i0 = 64; i0 < n; i0 += 64) {
+        a[2] = fetch(i0 + lane);
+        a[3] = fetch(i0 + lane + 32);
+        // bitonic over elements 32 t + lane
+#pragma unroll 1
+        for (uint32_t size = 2; size <= 128; size <<= 1) {
+#pragma unroll 1
+            for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
+                if (stride >= 32) {
+                    const bool far = stride == 64;
+                    const unsigned long long b0 = a[far ? 2 : 1], b1 = a[far ? 3 : 0];
+                    const unsigned long long b2 = a[far ? 0 : 3], b3 = a[far ? 1 : 2];
+                    const unsigned long long b[4] = {b0, b1, b2, b3};
+#pragma unroll
+                    for (uint32_t t = 0; t < 4; ++t) {
+                        const uint32_t e = 32 * t + lane;
+                        const bool low = ((e & size) == 0) == ((e & stride) == 0);
+                        a[t] = (b[t] < a[t]) == low ? b[t] : a[t];
+                    }
+                } else {
+#pragma unroll
+                    for (uint32_t t = 0; t < 4; ++t) {
+                        const unsigned long long b = __shfl_xor_sync(0xffffffffu, a[t], stride);
+                        const uint32_t e = 32 * t + lane;
+                        const bool low = ((e & size) == 0) == ((e & stride) == 0);
+                        a[t] = (b < a[t]) == low ? b : a[t];
+                    }
+                }
+            }
+        }
+    }
+    __syncwarp();  // every entry is read
+#pragma unroll
+    for (int t = 0; t < 2; ++t)
+        list[32 * t + lane] = make_uint2(__float_as_uint(key_to_float((uint32_t)(a[t] >> 32))), (uint32_t)a[t]);
+    __syncwarp();
+    return key_to_float((uint32_t)(__shfl_sync(0xffffffffu, a[1], 31) >> 32));
+}
 
 template <int MODE>
 __global__ __launch_bounds__(kThreads, 1) void k_tc_filter(const __grid_constant__ CUtensorMap tma_a,
@@ -213,7 +275,7 @@ __global__ __launch_bounds__(kThreads, 1) void k_tc_filter(const __grid_constant
             if (first >= p.pos1) continue;
             const uint32_t row = item / p.splits * 128u + quarter * 32u + lane;
             const bool in = row < p.M;
-            const float thr = MODE == kTcBelow && in ? p.thr[row] : -FLT_MAX;
+            float thr = MODE == kTcBelow && in ? p.thr[row] : -FLT_MAX;
             // this warp's part of the row's list: no other warp of the grid writes it
             const uint32_t part = item % p.splits * 2 + half;
             uint2* list = p.cand + (uint64_t)row * p.cap + part * p.seg;
@@ -310,10 +372,8 @@ __global__ __launch_bounds__(kThreads, 1) void k_tc_filter(const __grid_constant
                             if (gm[t] <= thr) {
 #pragma unroll
                                 for (int j = 8 * t; j < 8 * t + 8; ++j)
-                                    if (__uint_as_float(v[j]) <= thr && col + j < p.N) {
-                                        if (found < p.seg) list[found] = make_uint2(v[j], p.id0 + col + j);
-                                        ++found;
-                                    }
+                                    if (__uint_as_float(v[j]) <= thr && col + j < p.N)
+                                        list[found++] = make_uint2(v[j], p.id0 + col + j);
                             }
                     }
                     if (MODE == kTcDense && in) {
@@ -324,6 +384,22 @@ __global__ __launch_bounds__(kThreads, 1) void k_tc_filter(const __grid_constant
                             out[j] = make_uint2(v[j], col + j < p.N ? p.id0 + col + j : kNoLabel);
                     }
                     if (cg + 1 < kCols / 32) arrived(r[(cg + 1) & 1]);
+                    if (MODE == kTcBelow) {
+                        // parts without room for the entries of 32 more columns
+                        unsigned full = __ballot_sync(0xffffffffu, found + 32 > p.seg);
+                        while (full) {
+                            const int r = __ffs(full) - 1;
+                            full &= full - 1;
+                            const float t = cut_back(
+                                reinterpret_cast<uint2*>(__shfl_sync(
+                                    0xffffffffu, (unsigned long long)reinterpret_cast<uintptr_t>(list), r)),
+                                __shfl_sync(0xffffffffu, found, r));
+                            if (lane == r) {
+                                found = kTcFilterKeep;
+                                thr = t;
+                            }
+                        }
+                    }
                 }
                 // this accumulator may take the next tile's MMAs
                 asm volatile("tcgen05.fence::before_thread_sync;");
@@ -456,6 +532,7 @@ cudaError_t launch_tc_filter(int mode, const uint16_t* A, uint64_t a_rs, const u
     p.splits = tc_filter_splits(p.M);
     if (p.splits > p.pos1 - p.pos0) p.splits = p.pos1 - p.pos0;
     p.seg = p.cap / (2 * p.splits);
+    if (mode == kTcBelow && p.seg < kTcFilterPart) return cudaErrorInvalidValue;
     const uint32_t items = mt * p.splits, nch = (p.K + 63) / 64;
     const size_t smem = (size_t)a_buffers(nch) * nch * kABytes + kRing * kBBytes + 1024;
     const unsigned grid = items < sms ? items : sms;

@@ -1387,15 +1387,14 @@ constexpr int kSplitWarps = kSplitThreads / 32;
 constexpr int kSplitRec = PGPU_SPLIT_REC;    // record blocks per warp and step (il_bytes)
 static_assert(kSplitRec <= 4, "il_bytes has room for steps of 4 blocks");
 constexpr uint32_t kSplitMaxSlots = 512;     // probed clusters a split query may have
-constexpr uint32_t kSplitRows = 4096;        // floats of cell terms a group of clusters may take
 
 __host__ __device__ inline SplitLayout split_layout(uint32_t nsq, uint32_t d, uint32_t F, uint32_t P,
-                                                    uint32_t budget) {
+                                                    uint32_t budget, uint32_t rows) {
     SplitLayout y;
     const uint32_t maxl = P < kSplitMaxSlots ? P : kSplitMaxSlots;
     y.slots = il_table_bytes(false) + il_query_bytes(d);
     y.rows_per = (F + 3u) & ~3u;
-    y.group = kSplitRows / y.rows_per;
+    y.group = rows / y.rows_per;
     y.group = y.group < 1 ? 1 : (y.group > maxl ? maxl : y.group);
     y.srow = y.slots + (6u * 4u * (maxl + 1) + 15u) / 16u * 16u;
     y.keys = y.srow + y.group * y.rows_per * 4u;
@@ -1406,9 +1405,16 @@ __host__ __device__ inline SplitLayout split_layout(uint32_t nsq, uint32_t d, ui
     return y;
 }
 // Two blocks per SM when the buffer then takes T keys one and a half times over, else one.
+// rows: floats of cell terms that a group of clusters may take (one cluster's at least). A block
+// alone on its SM has room for more; with one cluster per group its eight warps wait for each
+// cluster's terms in turn: 2000 queries over 300 clusters of 200 records and 4096 fine ids
+// took 8.67 ms (8.28 with two blocks and every distance in memory), 6.83 with six clusters to a
+// group, 7.22 with four. The buffer keeps room for four times T: at T = 2000 more rows than
+// 16384 leave too few keys (500 clusters of 1000 records: 8.50 ms, 9.59 with 24576).
 // Either way the buffer has to take the first sampled keys and their select's histogram.
 constexpr uint32_t kSplitBudget2 = 111 * 1024, kSplitBudget1 = 220 * 1024;
 constexpr uint32_t kSplitLeast = kSplitSampleStep + kSplitHistKeys;
+constexpr uint32_t kSplitRows2 = 4096, kSplitRows1[] = {24576, 16384, kSplitRows2};
 static uint32_t split_need(uint32_t T) {
     const uint32_t n = T + T / 2 + 512;
     return n > kSplitLeast ? n : kSplitLeast;
@@ -1925,9 +1931,13 @@ cudaError_t launch_scan_order(const DeviceIndex& ix, uint32_t n, Scratch& s, cud
 }
 
 SplitLayout split_choice(const DeviceIndex& ix, uint32_t P, uint32_t T) {
-    const SplitLayout two = split_layout(ix.nsq, ix.d, ix.F, P, kSplitBudget2);
+    const SplitLayout two = split_layout(ix.nsq, ix.d, ix.F, P, kSplitBudget2, kSplitRows2);
     if (two.bytes && two.cap >= split_need(T)) return two;
-    const SplitLayout one = split_layout(ix.nsq, ix.d, ix.F, P, kSplitBudget1);
+    SplitLayout one{};
+    for (uint32_t rows : kSplitRows1) {
+        one = split_layout(ix.nsq, ix.d, ix.F, P, kSplitBudget1, rows);
+        if (one.bytes && one.cap >= 4 * T + kSplitLeast) return one;
+    }
     return one.bytes && one.cap >= T + 512 + kSplitLeast ? one : SplitLayout{};
 }
 

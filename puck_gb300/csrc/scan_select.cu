@@ -206,12 +206,9 @@ constexpr uint64_t kKeyMax = ~0ull;
 // select with 8-bit digits, stopping as soon as the chosen digit's bucket holds
 // one key (usually after the 2nd or 3rd digit of the float). `hist` has 256
 // slots, `sel` 4. All threads call it.
-// max_digits > 0 stops after that many digit passes and returns the largest key of
-// the bucket reached: then at least K keys are <= the result (a cut-back bound, not
-// the K-th itself).
 template <int NT>
 __device__ uint64_t block_select_kth(const uint64_t* keys, uint32_t count, uint32_t K,
-                                     uint32_t* hist, uint64_t* sel, int max_digits = 0) {
+                                     uint32_t* hist, uint64_t* sel) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // the leading bits every key shares need no pass: start at the digit where the
     // smallest and the largest key first differ
@@ -304,8 +301,6 @@ __device__ uint64_t block_select_kth(const uint64_t* keys, uint32_t count, uint3
         k = (uint32_t)sel[1];
         const bool unique = sel[2] == 1;
         __syncthreads();
-        if (!unique && max_digits > 0 && --max_digits == 0 && shift > 0)
-            return prefix | ~mask;
         if (unique && shift > 0) {
             // the one key under this prefix is the K-th
             for (uint32_t i = tid; i < count; i += NT)

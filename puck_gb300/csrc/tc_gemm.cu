@@ -3,8 +3,8 @@
 //   acc[i][j] = sum_k bf16(A(i,k)) * bf16(B(j,k))          (FP32 accumulation)
 //
 // A(i,k) = A.p[i*A.rs + k*A.ks], B(j,k) likewise: FP32 operands in any 2-D
-// layout (row-major, or transposed for the weight gradients of the probe
-// network). They are rounded to BF16 while being staged into shared memory in
+// layout (row-major, or transposed; the library's own operands are row-major,
+// strided ones come through pgpu_contract_bf16). They are rounded to BF16 while being staged into shared memory in
 // the canonical no-swizzle K-major layout of tcgen05: 8-row x 16-byte core
 // matrices, the 16 row groups of a 128-row tile 128 B apart (stride byte offset),
 // K groups of 8 elements 2 KiB apart (leading byte offset).

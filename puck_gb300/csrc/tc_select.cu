@@ -633,8 +633,9 @@ cudaError_t launch_coarse_window(const DeviceIndex& ix, uint32_t n, Scratch& s,
 }
 
 // nearest_center through the MINIMA screen (k_tc_filter) and k_group_argmin, in chunks whose
-// BF16 rows and group minima stay in L2 between the kernels; a call allocates 50 MB at most
-// beside the centroids' copies.
+// BF16 rows and group minima stay in L2 between the kernels; a call allocates 50 MB beside the
+// centroids' copies, more only above 0.75M centroids (a chunk has 128 rows at least, and a row
+// half a byte of minima per centroid: 1 GB at the limit of 2^24).
 static cudaError_t nearest_center_screened(uint32_t dim, const float* cents, uint32_t k, const float* x,
                                            uint64_t n, int32_t* assign, float* dis,
                                            cudaStream_t stream) {

@@ -353,7 +353,8 @@ __global__ __launch_bounds__(256) void k_window_small(
 // clusters are apart) are measured in the reference's FP32 order, lane = centroid; the smallest
 // cur_j with the lowest id wins, as in the reference's strict-< scan. Rows or centroids too
 // large for the bound, or a failed screen: every group. Eight lanes per point, four points per
-// warp; bound by the L2 and L1 traffic of the centroid rows, for which groups of 8 are read by
+// warp; bound by the centroid rows' loads (their latency, and L1 at two thirds of its rate; 13%
+// of the sectors hit there), for which groups of 8 are read by
 // the row (groups of 32 read as columns of a transposed copy took 135 us for 77824 points of 96
 // dimensions against 2000 centroids, groups of 8 so 160, this 90). The whole call on 262144 such
 // points: 3.57 ms with a screen matrix in memory, 0.60 now; 131072 points of 4 dimensions

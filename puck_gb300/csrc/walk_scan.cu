@@ -39,7 +39,8 @@
 //     max_stat, or rank 0 breaks) are passed over a block's width at a time.
 // Measured on a GB300, whole calls: one query over 200k points with filter_topk 1100 (57k
 // records and 3.4k inserts) 9.9 ms with a one-thread replay, 2.7 ms now; 10k queries over 1M
-// points with filter_topk 200 15.1 ms, now 8.4 ms (the walk itself 10.9 and 4.4 ms).
+// points with filter_topk 200 15.1 ms, now 6.7 ms (the walk itself 10.9 and 4.4 ms, where three
+// of a block's four warps wait at its barrier for the replay: 19% of the issue slots are used).
 #include "device_common.cuh"
 #include "pgpu_internal.h"
 

@@ -16,7 +16,7 @@
 // below a query's threshold; the filter cuts a full part of a list back to its 64
 // smallest. Dimensions above the filter's limit: launch_knn_dense, with the screen
 // matrix in memory.
-// 2048 queries of 96 dimensions over 1M points: 2.05 ms (2.7 in the order of their clusters),
+// 2048 queries of 96 dimensions over 1M points: 2.08 ms (3.5 in the order of their clusters),
 // against 24.5 ms with the screen matrix in memory. The tensor filter's passes are 1.1 ms of it,
 // the lists' merges 0.23.
 #include <algorithm>
@@ -336,12 +336,9 @@ cudaError_t launch_knn(const float* base, uint64_t n, uint32_t d, const float* Q
     // base rows held in BF16 at a time: 256 MiB, whole tiles
     uint64_t held = (256ull << 20) / (2ull * dp) / kTcFilterTile * kTcFilterTile;
     if (held > n) held = n;
-    const uint32_t tiles_held = (uint32_t)((held + kTcFilterTile - 1) / kTcFilterTile);
-    const uint64_t padded = (uint64_t)tiles_held * kTcFilterTile;
+    const uint64_t padded = (held + kTcFilterTile - 1) / kTcFilterTile * kTcFilterTile;
     // list entries per query: the first columns, or the least that each part takes
-    auto cap_of = [tiles_held](uint32_t rows) {
-        return std::max(2048u, 2 * kTcFilterPart * std::min(tc_filter_splits(rows), tiles_held));
-    };
+    auto cap_of = [](uint32_t rows) { return std::max(2048u, 2 * kTcFilterKeep * tc_filter_splits(rows)); };
     const uint32_t last = nq % kQC ? nq % kQC : qc;  // rows of the last chunk of queries
     uint64_t bytes = 0;
     auto part = [&](uint64_t size) {

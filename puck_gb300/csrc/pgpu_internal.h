@@ -357,8 +357,7 @@ cudaError_t launch_tc_gemm(const TcOperand& A, const TcOperand& B, uint32_t K,
                            const TcEpilogue& ep, int* err, cudaStream_t stream);
 // Contraction with a selecting epilogue (tc_filter.cu): s_ij = bias_j - a_i.b_j over BF16 rows.
 constexpr uint32_t kTcFilterTile = 256;  // columns per tile
-constexpr uint32_t kTcFilterKeep = 64;   // BELOW: entries a part keeps when it is cut back
-constexpr uint32_t kTcFilterPart = kTcFilterKeep + 32;  // the least a part takes
+constexpr uint32_t kTcFilterKeep = 64;   // BELOW: entries a part takes at least, and keeps when cut back
 enum { kTcMinima = 0, kTcBelow = 1, kTcDense = 2 };
 struct TcFilter {
     uint32_t M, N, K;          // rows of A and B, dimensions (tc_filter_applies)

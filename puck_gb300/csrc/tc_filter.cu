@@ -8,10 +8,10 @@
 //   BELOW   the (score, column) pairs at or below a row's threshold, in its list: the screen of
 //           the brute-force neighbours. A row's list has a part for each warp that works on the
 //           row, so an entry costs no atomic (one with its result on the way took 3 of the 6 ms
-//           of a million columns). A part that may not take 32 more columns' entries is cut
-//           back to its kTcFilterKeep smallest, which are all that the row's smallest can need of it, and
-//           the last of them is the row's threshold there: no order of the columns overflows a
-//           list. DENSE fills the lists for the first columns.
+//           of a million columns). A part that cannot take the entries of 32 more columns is
+//           cut back, with them, to its kTcFilterKeep smallest, which are all that the row's smallest
+//           can need of it, and the last of them is the row's threshold there: no order of the
+//           columns overflows a list. DENSE fills the lists for the first columns.
 //
 // One CTA per SM loops over items, an item being a 128-row tile of A and every splits-th of a
 // range of 256-column tiles of B (position p stands for tile (p * step) mod tiles: a range of
@@ -51,15 +51,15 @@ constexpr uint32_t kABytes = 128u * 64u * 2u, kBBytes = kNT * 64u * 2u;
 // A tiles held: two where they fit beside the ring.
 __host__ __device__ constexpr uint32_t a_buffers(uint32_t nch) { return nch <= 2 ? 2u : 1u; }
 
-// A part of a list cut back to its kTcFilterKeep smallest (score, column), by one warp: kept keys
-// sorted in registers (0 and 1; two per lane), the rest brought in 64 at a time (2 and 3) and the
-// 128 sorted. Returns the largest score kept. n > kTcFilterKeep entries. Asked for after every 32
-// columns, so that a part needs room for 96 entries and no more memory than without: one million
-// rows in the order of 1024 clusters, 2048 queries, take 2.7 ms (28 where an overflowing part had
-// the call repeated with the screen in memory), shuffled 2.16 (2.23). Asked after 128 columns
-// the larger parts cost 30 to 90 us of allocation; one thread replacing the largest of its full
-// part took 9.3 ms.
-__device__ __noinline__ float cut_back(uint2* list, uint32_t n) {
+// A part of a list, n entries, and up to 32 new ones (a key per lane, ~0: none) cut back to the
+// kTcFilterKeep smallest (score, column) by one warp: the smallest so far sorted in registers (0
+// and 1; two per lane), the rest brought in 64 at a time (2 and 3) and the 128 sorted. Returns the
+// largest score kept. More than kTcFilterKeep entries in all. The new ones come from registers, so
+// that a part needs room for the kept ones alone and a call no more memory than without (it is
+// allocated by the call, and each further 32 MB of it cost 130 us): one million rows in the order
+// of 1024 clusters, 2048 queries, take 3.5 ms (28 where an overflowing part had the call repeated
+// with the screen in memory). One thread replacing the largest of its full part took 9.3 ms.
+__device__ __forceinline__ float cut_back(uint2* list, uint32_t n, unsigned long long extra) {
     static_assert(kTcFilterKeep == 64, "two keys per lane");
     const uint32_t lane = threadIdx.x & 31;
     __syncwarp();  // the lane that wrote the entries is another
@@ -71,9 +71,10 @@ __device__ __noinline__ float cut_back(uint2* list, uint32_t n) {
     };
     a[0] = fetch(lane);
     a[1] = fetch(lane + 32);
-    for (uint32_t i0 = 64; i0 < n; i0 += 64) {
-        a[2] = fetch(i0 + lane);
-        a[3] = fetch(i0 + lane + 32);
+    for (uint32_t i0 = 64;; i0 += 64) {
+        const bool last = i0 >= n;
+        a[2] = last ? extra : fetch(i0 + lane);
+        a[3] = last ? ~0ull : fetch(i0 + lane + 32);
         // bitonic over elements 32 t + lane
 #pragma unroll 1
         for (uint32_t size = 2; size <= 128; size <<= 1) {
@@ -101,6 +102,7 @@ __device__ __noinline__ float cut_back(uint2* list, uint32_t n) {
                 }
             }
         }
+        if (last) break;
     }
     __syncwarp();  // every entry is read
 #pragma unroll
@@ -367,13 +369,47 @@ __global__ __launch_bounds__(kThreads, 1) void k_tc_filter(const __grid_constant
                     }
                     const uint32_t col = n0 + cg * 32;
                     if (MODE == kTcBelow) {
+                        float lim = thr;
+                        if (__any_sync(0xffffffffu, found + 32 > p.seg)) {
+                            // a part may not take these columns' entries: look who has how many
+                            // (first the load under way: this path may move registers)
+                            if (cg + 1 < kCols / 32) arrived(r[(cg + 1) & 1]);
+                            uint32_t hits = 0;
+#pragma unroll
+                            for (int j = 0; j < 32; ++j)
+                                hits |= (__uint_as_float(v[j]) <= thr && col + j < p.N ? 1u : 0u) << j;
+                            unsigned over = __ballot_sync(0xffffffffu, found + __popc(hits) > p.seg);
+                            while (over) {
+                                const int r0 = __ffs(over) - 1;
+                                over &= over - 1;
+                                uint32_t x = 0;  // that row's score of column `lane`
+#pragma unroll
+                                for (int j = 0; j < 32; ++j) {
+                                    const uint32_t u = __shfl_sync(0xffffffffu, v[j], r0);
+                                    x = lane == j ? u : x;
+                                }
+                                const bool hit = __shfl_sync(0xffffffffu, hits, r0) >> lane & 1u;
+                                const float t = cut_back(
+                                    reinterpret_cast<uint2*>(__shfl_sync(
+                                        0xffffffffu, (unsigned long long)reinterpret_cast<uintptr_t>(list), r0)),
+                                    __shfl_sync(0xffffffffu, found, r0),
+                                    hit ? ((unsigned long long)ordered_key(__uint_as_float(x) + 0.0f) << 32) |
+                                              (p.id0 + col + lane)
+                                        : ~0ull);
+                                if (lane == r0) {
+                                    found = kTcFilterKeep;
+                                    thr = t;
+                                    lim = __int_as_float(0x7fffffff);  // these columns are done
+                                }
+                            }
+                        }
                         // entries are rare: eight columns with one are looked through
 #pragma unroll
                         for (int t = 0; t < 4; ++t)
-                            if (gm[t] <= thr) {
+                            if (gm[t] <= lim) {
 #pragma unroll
                                 for (int j = 8 * t; j < 8 * t + 8; ++j)
-                                    if (__uint_as_float(v[j]) <= thr && col + j < p.N)
+                                    if (__uint_as_float(v[j]) <= lim && col + j < p.N)
                                         list[found++] = make_uint2(v[j], p.id0 + col + j);
                             }
                     }
@@ -385,22 +421,6 @@ __global__ __launch_bounds__(kThreads, 1) void k_tc_filter(const __grid_constant
                             out[j] = make_uint2(v[j], col + j < p.N ? p.id0 + col + j : kNoLabel);
                     }
                     if (cg + 1 < kCols / 32) arrived(r[(cg + 1) & 1]);
-                    if (MODE == kTcBelow) {
-                        // parts without room for the entries of 32 more columns
-                        unsigned full = __ballot_sync(0xffffffffu, found + 32 > p.seg);
-                        while (full) {
-                            const int r = __ffs(full) - 1;
-                            full &= full - 1;
-                            const float t = cut_back(
-                                reinterpret_cast<uint2*>(__shfl_sync(
-                                    0xffffffffu, (unsigned long long)reinterpret_cast<uintptr_t>(list), r)),
-                                __shfl_sync(0xffffffffu, found, r));
-                            if (lane == r) {
-                                found = kTcFilterKeep;
-                                thr = t;
-                            }
-                        }
-                    }
                 }
                 // this accumulator may take the next tile's MMAs
                 asm volatile("tcgen05.fence::before_thread_sync;");
@@ -533,7 +553,7 @@ cudaError_t launch_tc_filter(int mode, const uint16_t* A, uint64_t a_rs, const u
     p.splits = tc_filter_splits(p.M);
     if (p.splits > p.pos1 - p.pos0) p.splits = p.pos1 - p.pos0;
     p.seg = p.cap / (2 * p.splits);
-    if (mode == kTcBelow && p.seg < kTcFilterPart) return cudaErrorInvalidValue;
+    if (mode == kTcBelow && p.seg < kTcFilterKeep) return cudaErrorInvalidValue;
     const uint32_t items = mt * p.splits, nch = (p.K + 63) / 64;
     const size_t smem = (size_t)a_buffers(nch) * nch * kABytes + kRing * kBBytes + 1024;
     const unsigned grid = items < sms ? items : sms;
